@@ -62,7 +62,7 @@ def _stale(out: Path, deps: list[Path]) -> bool:
 
 
 def _headers() -> list[Path]:
-    return list(CSRC.glob("*.h")) + list((ROOT / "include").rglob("*.h"))
+    return list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + list((ROOT / "include").rglob("*.h"))
 
 
 def build_library(verbose: bool = False) -> Path:
