@@ -1,0 +1,294 @@
+// fp64_alu.cuh -- FP64 square root, division and product on the integer
+// units, correctly rounded (round to nearest even): the bits of the IEEE
+// operation, which is what the FP64 form's parity with the CPU oracle needs.
+//
+// Why: GB300 executes 1.6 FP64 operations per SM and clock (measured, any of
+// add, multiply, fma, compare or conversion: a warp instruction takes 20
+// cycles of the SM), against 23 32x32->64-bit multiply-adds, 60 logic
+// operations or shifts and 118 additions.  A square root or a division is
+// eight or more FP64 instructions (160 cycles a warp); below, a division by
+// a divisor whose reciprocal is at hand is about 13 cycles and a product
+// about 12, and they leave the FP64 pipe to the additions.  Measured, entry
+// forces with square root, divisions and products here against all on the
+// FP64 pipe, per step: 70^3 lattice 0.93 -> 0.48 ms, 96 bodies of 3-9 masses
+// per side 87 -> 49 us, a 24x19x27 block with RK2 99 -> 55 us.
+//
+// Method: operands are split into a 53-bit integer significand and an
+// exponent.  The square root and the quotient are integers Q with a known
+// exact remainder condition: an estimate from a reciprocal (square root)
+// good to about 2^-59 -- a 22-bit FP32 hardware estimate improved by one
+// third-order step, y (1 + e/2 + 3 e^2/8) with e = 1 - n y^2, or y (1 + e +
+// e^2) with e = 1 - n y (over all FP32 significands |e| < 2^-20.8 and
+// 2^-21.8 on the GPU, so what the step leaves out is below 2^-64) -- gives Q to within a little more than half a unit,
+// biased down, and the exact remainder modulo 2^64 (it is far smaller than
+// 2^63 in magnitude) says whether the next integer is nearer.  Neither a
+// quotient nor a square root of 53-bit operands can lie half-way between two
+// 53-bit numbers, so no tie arises; a product's does, and is rounded from
+// its exact 106 bits.
+//
+// Range: operands are normal with exponents in [2^-250, 2^250], or zero (an
+// exponent of kAluZero, carried through products and quotients: a result
+// with a negative exponent is a zero).  alu_unpack reports anything else
+// (subnormals, infinities, NaN, huge and tiny values) in `bad`; the caller
+// then uses the FP64 instructions.
+//
+// The host compiles the same functions (with its own initial estimates), so
+// that they are also tested on the CPU.
+#pragma once
+
+#include <cstdint>
+#include <cstring>
+
+#ifdef __CUDACC__
+#define TG_HD __host__ __device__ __forceinline__
+#else
+#include <cmath>
+#define TG_HD inline
+#endif
+
+namespace tg {
+
+constexpr int kAluZero = -100000;  // exponent of a zero
+constexpr int kAluLo = 1023 - 250, kAluHi = 1023 + 250;
+
+// value = (-1)^sign * m * 2^(e - 1075), m in [2^52, 2^53); e <= 0: zero
+struct Alu {
+    uint64_t m;
+    int e;
+    uint32_t sign;  // 0 or 0x80000000
+};
+
+TG_HD uint64_t alu_bits(double x) {
+#ifdef __CUDA_ARCH__
+    return (uint64_t)__double_as_longlong(x);
+#else
+    uint64_t b;
+    std::memcpy(&b, &x, 8);
+    return b;
+#endif
+}
+TG_HD double alu_double(uint64_t b) {
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)b);
+#else
+    double x;
+    std::memcpy(&x, &b, 8);
+    return x;
+#endif
+}
+TG_HD uint64_t alu_join(uint32_t hi, uint32_t lo) { return ((uint64_t)hi << 32) | lo; }
+TG_HD uint32_t alu_lo(uint64_t x) { return (uint32_t)x; }
+TG_HD uint32_t alu_hi(uint64_t x) { return (uint32_t)(x >> 32); }
+TG_HD uint64_t alu_mad(uint32_t a, uint32_t b, uint64_t c) { return (uint64_t)a * b + c; }  // one IMAD.WIDE
+TG_HD uint32_t alu_mulhi(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+    return __umulhi(a, b);
+#else
+    return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+// the low 32 bits of (hi : lo) >> s, s < 32
+TG_HD uint32_t alu_shr(uint32_t lo, uint32_t hi, uint32_t s) {
+#ifdef __CUDA_ARCH__
+    return __funnelshift_r(lo, hi, s);
+#else
+    return (uint32_t)(((((uint64_t)hi) << 32) | lo) >> s);
+#endif
+}
+// the high 64 bits of a 64 x 64 product, at most 3 too small
+TG_HD uint64_t alu_mulhi64(uint64_t a, uint64_t b) {
+    return alu_mad(alu_hi(a), alu_hi(b), (uint64_t)alu_mulhi(alu_hi(a), alu_lo(b)) + alu_mulhi(alu_lo(a), alu_hi(b)));
+}
+// the low 64 bits of a 64 x 64 product
+TG_HD uint64_t alu_mullo64(uint64_t a, uint64_t b) {
+    const uint64_t p = (uint64_t)alu_lo(a) * alu_lo(b);
+    return alu_join(alu_hi(p) + alu_lo(a) * alu_hi(b) + alu_hi(a) * alu_lo(b), alu_lo(p));
+}
+// 1/sqrt(x), 1/x, good to 22 bits
+TG_HD float alu_rsqrt_estimate(float x) {
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+#else
+    return 1.0f / std::sqrt(x);
+#endif
+}
+TG_HD float alu_rcp_estimate(float x) {
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+#else
+    return 1.0f / x;
+#endif
+}
+TG_HD uint32_t alu_float_bits(float x) {
+#ifdef __CUDA_ARCH__
+    return __float_as_uint(x);
+#else
+    uint32_t b;
+    std::memcpy(&b, &x, 4);
+    return b;
+#endif
+}
+TG_HD float alu_float(uint32_t b) {
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(b);
+#else
+    float x;
+    std::memcpy(&x, &b, 4);
+    return x;
+#endif
+}
+
+TG_HD Alu alu_unpack(double x, bool &bad) {
+    const uint64_t b = alu_bits(x);
+    const uint32_t h = alu_hi(b);
+    Alu a;
+    a.sign = h & 0x80000000u;
+    a.e = (int)((h >> 20) & 0x7ffu);
+    a.m = alu_join((h & 0xfffffu) | 0x100000u, alu_lo(b));
+    const bool in = (uint32_t)(a.e - kAluLo) <= (uint32_t)(kAluHi - kAluLo);
+    const bool zero = ((h << 1) | alu_lo(b)) == 0;
+    bad |= !(in || zero);
+    if (zero) a.e = kAluZero;
+    return a;
+}
+
+TG_HD double alu_pack(const Alu &a) {
+    // m's top bit adds one to the exponent field
+    const uint32_t h = alu_hi(a.m) + ((uint32_t)(a.e - 1) << 20);
+    const bool nz = a.e > 0;
+    return alu_double(alu_join((nz ? h : 0u) | a.sign, nz ? alu_lo(a.m) : 0u));
+}
+
+// m = 2^53 (a significand rounded up over the top) becomes 2^52
+TG_HD void alu_carry(Alu &a) {
+    const uint32_t c = alu_hi(a.m) >> 21;
+    a.m >>= c;
+    a.e += (int)c;
+}
+
+// The product's 106 bits hi : w rounded to 53: hi in [2^52, 2^54), w the 32
+// bits below it with a sticky lowest bit.
+TG_HD Alu alu_round(uint64_t hi, uint32_t w, int e, uint32_t sign) {
+    const uint32_t s = alu_hi(hi) >> 21;  // 1: hi has 54 bits
+    const uint32_t h = alu_hi(hi) >> s, l = alu_shr(alu_lo(hi), alu_hi(hi), s);
+    // below the half-way bit: the sticky bit, and l's lowest (half-way cases
+    // go to the even neighbour)
+    w = alu_shr(w, alu_lo(hi), s) | ((w | l) & 1u);
+    Alu r;
+    r.m = alu_join(h, l) + (w > 0x80000000u ? 1u : 0u);
+    r.e = e + (int)s;
+    r.sign = sign;
+    return r;
+}
+
+// a * b; the result's m may be 2^53 (alu_pack takes that; alu_carry for
+// further use as an operand)
+TG_HD Alu alu_mul(const Alu &a, const Alu &b) {
+    const uint64_t x = a.m << 1, y = b.m << 11;
+    const uint32_t xl = alu_lo(x), xh = alu_hi(x), yl = alu_lo(y), yh = alu_hi(y);
+    const uint64_t p = alu_mad(xl, yl, 0);
+    const uint64_t t = alu_mad(xl, yh, alu_hi(p));
+    const uint64_t u = alu_mad(xh, yl, alu_lo(t));
+    const uint64_t hi = alu_mad(xh, yh, (uint64_t)alu_hi(t)) + alu_hi(u);
+    const uint32_t w = alu_lo(u) | (alu_lo(p) != 0 ? 1u : 0u);
+    return alu_round(hi, w, a.e + b.e - 1023, a.sign ^ b.sign);
+}
+
+TG_HD Alu alu_square(const Alu &a) {
+    const uint64_t x = a.m << 6;  // 59 bits: x^2 = m^2 2^12
+    const uint32_t xl = alu_lo(x), xh = alu_hi(x);
+    const uint64_t p = alu_mad(xl, xl, 0);
+    const uint64_t t = alu_mad(xl, xh << 1, alu_hi(p));  // xh < 2^27
+    const uint64_t hi = alu_mad(xh, xh, (uint64_t)alu_hi(t));
+    const uint32_t w = alu_lo(t) | (alu_lo(p) != 0 ? 1u : 0u);
+    return alu_round(hi, w, 2 * a.e - 1023, 0);
+}
+
+// A divisor: significand, exponent and reciprocal, r = 2^115 / m (2^62 <= r
+// <= 2^63), relative error below 2^-58.5.
+struct AluDivisor {
+    uint64_t m, r;
+    int e;
+    uint32_t sign;
+};
+
+// a / d; the result's m may be 2^53
+TG_HD Alu alu_div(const Alu &a, const AluDivisor &d) {
+    const uint64_t t = alu_mulhi64(a.m << 11, d.r);  // (a.m / d.m) 2^62, within 24
+    const uint32_t s = (alu_hi(t) >> 30) ^ 1u;       // 0: a.m >= d.m, 53 bits are t >> 10; 1: t >> 9
+    // nearest integer from below: 64 units of 2^9 or 2^10 short of half
+    uint64_t q = (t + ((512u >> s) - 64u)) >> (10 - s);
+    // exact remainder a.m 2^(52+s) - q d.m
+    const uint64_t num = alu_join(alu_lo(a.m) << (20 + s), 0);
+    const uint64_t rem = num - alu_mullo64(q, d.m);
+    const uint64_t x = d.m - (rem << 1);
+    q += alu_hi(x) >> 31;
+    return Alu{q, a.e - d.e + 1023 - (int)s, a.sign ^ d.sign};
+}
+
+// |x| as a divisor from its unpacked form (not zero)
+TG_HD AluDivisor alu_divisor(const Alu &x) {
+    // y23 2^-23 = 1/v, v = m 2^-52 in [1, 2)
+    const float v = alu_float(0x3f800000u | alu_lo(x.m >> 29));  // m's bit 52 lands on exponent bit 0, set already
+    const uint32_t y = alu_float_bits(alu_rcp_estimate(v) + 1.0f) - 0x3f800000u;
+    // e = 1 - v y: m y in units of 2^-75 -> keep 2^-64 (modulo 1: |e| < 2^-19)
+    const uint64_t lo = (uint64_t)alu_lo(x.m) * y;
+    const uint64_t prod_hi = alu_mad(alu_hi(x.m), y, lo >> 32);  // units of 2^-43
+    const uint64_t e64 = 0 - ((prod_hi << 21) | (alu_lo(lo) >> 11));
+    const int64_t e = (int64_t)e64;
+    const int32_t et = (int32_t)(e >> 16);                          // units of 2^-48
+    const uint32_t et_abs = (uint32_t)(et < 0 ? -et : et);
+    const uint32_t e2 = alu_mulhi(et_abs, et_abs);                  // e^2, units of 2^-64
+    const uint64_t c = e64 + e2;                                    // e + e^2, 2^-64
+    // r = 2^63 y23 2^-23 (1 + c)
+    const uint64_t yc = ((uint64_t)y * alu_lo(c)) >> 24;            // 2^63 2^-23 2^-64 = 2^-24
+    const int64_t yh = (int64_t)(int32_t)alu_hi(c) * (int32_t)y;    // times 2^32: << 8
+    return AluDivisor{x.m, ((uint64_t)y << 40) + (uint64_t)(yh * 256) + yc, x.e, x.sign};
+}
+
+// sqrt of the positive number n, and the result as a divisor
+TG_HD Alu alu_sqrt(const Alu &n, AluDivisor &d) {
+    // n = N 2^(2h), N in [2^52, 2^54)
+    const uint32_t odd = (uint32_t)(n.e - 1075) & 1u;
+    const uint64_t N = n.m << odd;
+    const int h = (n.e - 1075 - (int)odd) >> 1;
+    // y 2^-23 = 1/sqrt(N 2^-52)
+    const float v = alu_float((0x3f800000u + (odd << 23)) | (alu_lo(n.m >> 29) & 0x7fffffu));
+    const uint32_t y = alu_float_bits(alu_rsqrt_estimate(v) + 1.0f) - 0x3f800000u;
+    // e = 1 - N y^2, in units of 2^-66 modulo 2^64 (|e| < 2^-19)
+    const uint64_t P = (uint64_t)y * y;
+    uint64_t t = alu_mad(alu_hi(N), alu_lo(P), alu_mulhi(alu_lo(N), alu_lo(P)));
+    t = alu_mad(alu_lo(N), alu_hi(P), t);
+    t += (uint64_t)(alu_hi(N) * alu_hi(P)) << 32;
+    const int64_t e = (int64_t)(0 - t);
+    const int32_t et = (int32_t)(e >> 16);                       // units of 2^-50
+    const uint32_t et_abs = (uint32_t)(et < 0 ? -et : et);
+    const uint32_t e2 = alu_mulhi(et_abs, et_abs);               // e^2, units of 2^-68
+    const int64_t c = (e >> 1) + ((e2 * 3u) >> 5);               // e/2 + 3 e^2/8, 2^-66
+    // y63 = 2^63 y 2^-23 (1 + c)
+    const uint64_t cl = ((uint64_t)y * alu_lo((uint64_t)c)) >> 26;
+    const int64_t ch = (int64_t)(int32_t)alu_hi((uint64_t)c) * (int32_t)y;  // times 2^32: << 6
+    const uint64_t y63 = ((uint64_t)y << 40) + (uint64_t)(ch * 64) + cl;
+    // S = sqrt(N 2^52) from below, then the exact remainder N 2^52 - S^2
+    const uint64_t sx = alu_mulhi64(N << 10, y63);               // sqrt(N 2^-52) 2^61
+    uint64_t S = (sx + (256u - 64u)) >> 9;
+    const uint64_t p = (uint64_t)alu_lo(S) * alu_lo(S);
+    const uint64_t sq = alu_join(alu_hi(p) + alu_lo(S) * (alu_hi(S) << 1), alu_lo(p));
+    uint64_t rho = alu_join(alu_lo(N) << 20, 0) - sq;
+    const uint32_t up = alu_hi(S - rho) >> 31;                   // rho > S: S + 1 is nearer
+    rho -= up ? ((S << 1) | 1u) : 0;
+    S += up;
+    // 1/S = 1/sqrt(N 2^52) (1 + rho / (2 S^2)): rho y^3 2^-42 in y63's units
+    const uint32_t y16 = alu_hi(y63) >> 15;
+    const uint32_t y3 = (((y16 * y16) >> 16) * y16) >> 16;  // y16 = 2^16 where y = 1
+    const int32_t corr = ((int32_t)alu_hi(rho) * (int32_t)(y3 >> 7)) >> 19;
+    const int es = h - 26 + 1075;
+    d = AluDivisor{S, y63 + (uint64_t)(int64_t)corr, es, 0};
+    return Alu{S, es, 0};
+}
+
+}  // namespace tg

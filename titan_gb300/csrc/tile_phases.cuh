@@ -16,6 +16,7 @@
 #pragma once
 
 #include "engine.h"
+#include "fp64_alu.cuh"
 #include "state.cuh"
 #include "step_math.cuh"
 
@@ -95,6 +96,66 @@ struct F3 {
     typename Real<PREC>::T x, y, z;
 };
 
+// FP64 force with the FP64 instructions alone, for operands outside the range
+// of the integer-unit functions (fp64_alu.cuh).
+__device__ __noinline__ F3<P_FP64> spring_force_f64_wide(int sa, int sb, double k, double rs, double damping,
+                                                         const uint8_t *st) {
+    const double2 *pa = reinterpret_cast<const double2 *>(st + (int64_t)sa * 48);
+    const double2 *pb = reinterpret_cast<const double2 *>(st + (int64_t)sb * 48);
+    const double2 a0 = pa[0], a1 = pa[1], b0 = pb[0], b1 = pb[1];
+    const double d0 = b0.x - a0.x, d1 = b0.y - a0.y, d2 = b1.x - a1.x;
+    const double nrm = nrm3(d0, d1, d2);
+    const double u0 = d0 / nrm, u1 = d1 / nrm, u2 = d2 / nrm;
+    const double fs = k * (rs - nrm);
+    double f0 = u0 * fs, f1 = u1 * fs, f2 = u2 * fs;
+    if (damping != 0.0) {
+        const double2 a2 = pa[2], b2 = pb[2];
+        const double w0 = a1.y - b1.y, w1 = a2.x - b2.x, w2 = a2.y - b2.y;
+        const double dd = ((w0 * u0 + w1 * u1) + w2 * u2) * damping;
+        f0 = f0 + u0 * dd;
+        f1 = f1 + u1 * dd;
+        f2 = f2 + u2 * dd;
+    }
+    return F3<P_FP64>{f0, f1, f2};
+}
+
+// FP64 force: the reference's operations in the reference's order, the
+// additions on the FP64 pipe, the square root, divisions and products on the
+// integer units (fp64_alu.cuh: the same bits).
+__device__ __forceinline__ F3<P_FP64> spring_force_f64(int sa, int sb, double k, double rs, double damping,
+                                                       const uint8_t *st) {
+    const double2 *pa = reinterpret_cast<const double2 *>(st + (int64_t)sa * 48);
+    const double2 *pb = reinterpret_cast<const double2 *>(st + (int64_t)sb * 48);
+    const double2 a0 = pa[0], a1 = pa[1], b0 = pb[0], b1 = pb[1];
+    bool bad = false;
+    const Alu d0 = alu_unpack(b0.x - a0.x, bad), d1 = alu_unpack(b0.y - a0.y, bad),
+              d2 = alu_unpack(b1.x - a1.x, bad);
+    const Alu n2 = alu_unpack((alu_pack(alu_square(d0)) + alu_pack(alu_square(d1))) + alu_pack(alu_square(d2)), bad);
+    bad |= n2.e <= 0;
+    AluDivisor nd;
+    const double nrm = alu_pack(alu_sqrt(n2, nd));
+    Alu fs = alu_mul(alu_unpack(k, bad), alu_unpack(rs - nrm, bad));
+    alu_carry(fs);
+    Alu u0 = alu_div(d0, nd), u1 = alu_div(d1, nd), u2 = alu_div(d2, nd);
+    alu_carry(u0);
+    alu_carry(u1);
+    alu_carry(u2);
+    double f0 = alu_pack(alu_mul(u0, fs)), f1 = alu_pack(alu_mul(u1, fs)), f2 = alu_pack(alu_mul(u2, fs));
+    if (damping != 0.0) {
+        const double2 a2 = pa[2], b2 = pb[2];
+        const double w0 = alu_pack(alu_mul(alu_unpack(a1.y - b1.y, bad), u0)),
+                     w1 = alu_pack(alu_mul(alu_unpack(a2.x - b2.x, bad), u1)),
+                     w2 = alu_pack(alu_mul(alu_unpack(a2.y - b2.y, bad), u2));
+        Alu dd = alu_mul(alu_unpack((w0 + w1) + w2, bad), alu_unpack(damping, bad));
+        alu_carry(dd);
+        f0 = f0 + alu_pack(alu_mul(u0, dd));
+        f1 = f1 + alu_pack(alu_mul(u1, dd));
+        f2 = f2 + alu_pack(alu_mul(u2, dd));
+    }
+    if (bad) return spring_force_f64_wide(sa, sb, k, rs, damping, st);
+    return F3<P_FP64>{f0, f1, f2};
+}
+
 // Force on the right end of a spring whose ends are the state records sa
 // (left) and sb (right) staged at st; k, rest, damping from the spring's
 // record, type from its entry word, act its actuation record.
@@ -104,32 +165,16 @@ __device__ __forceinline__ F3<PREC> spring_force(int sa, int sb, uint32_t type, 
                                                  bool actuated, const Rec16<PREC> &act, const uint8_t *st,
                                                  const StepTime &t) {
     if constexpr (PREC == P_FP64) {
-        double scale = 1.0;
+        double rs = rest;  // rest * scale; a scale of 1 changes nothing
         if (actuated) {
             const double2 q01 = act.lo;
             const double2 q23 = act.hi;
             double th = q01.x * t.T;
             th = th + q23.x;
             const double sn = q01.y * sin(th);
-            scale = type == 2 ? 1.0 - sn : 1.0 + sn;
+            rs = rest * (type == 2 ? 1.0 - sn : 1.0 + sn);
         }
-        const double2 *pa = reinterpret_cast<const double2 *>(st + (int64_t)sa * 48);
-        const double2 *pb = reinterpret_cast<const double2 *>(st + (int64_t)sb * 48);
-        const double2 a0 = pa[0], a1 = pa[1], b0 = pb[0], b1 = pb[1];
-        const double d0 = b0.x - a0.x, d1 = b0.y - a0.y, d2 = b1.x - a1.x;
-        const double nrm = nrm3(d0, d1, d2);
-        const double u0 = d0 / nrm, u1 = d1 / nrm, u2 = d2 / nrm;
-        const double fs = k * (rest * scale - nrm);
-        double f0 = u0 * fs, f1 = u1 * fs, f2 = u2 * fs;
-        if (damping != 0.0) {
-            const double2 a2 = pa[2], b2 = pb[2];
-            const double w0 = a1.y - b1.y, w1 = a2.x - b2.x, w2 = a2.y - b2.y;
-            const double dd = ((w0 * u0 + w1 * u1) + w2 * u2) * damping;
-            f0 = f0 + u0 * dd;
-            f1 = f1 + u1 * dd;
-            f2 = f2 + u2 * dd;
-        }
-        return F3<PREC>{f0, f1, f2};
+        return spring_force_f64(sa, sb, k, rs, damping, st);
     } else {
         (void)type;
         float rs = rest;
