@@ -72,3 +72,32 @@ def test_pair_forces_bitwise(kind, kernel):
         seen &= np.repeat((sc["damping"] != 0) | (((pos[1::2] - pos[0::2]) ** 2).sum(1) > 0), 2)
     for got, want in ((st["acc"], o.acc), (st["vel"], o.vel), (st["pos"], o.pos)):
         assert np.array_equal(got[seen], want[seen], equal_nan=True)
+
+
+@pytest.mark.parametrize("lo,hi", [(-40, -20), (-12, 12), (26, 34)])
+def test_actuated_rest_length(lo, hi):
+    """The sine of actuated rest lengths: angles below, inside and above the
+    integer path's range (2^-24 to 2^30), both actuation types, amplitudes on
+    either side of its limit of 4.  A spring at rest length 1 whose ends are 1
+    apart has the force k (scale - 1), whose error against libm's sine is
+    bounded by the two sines' errors (below 2 units in the last place each)
+    and the roundings of amp sin and 1 -+ amp sin."""
+    rng = np.random.default_rng(100 + hi)
+    pairs = 3001
+    n = 2 * pairs
+    pos = np.zeros((n, 3))
+    pos[:, 1] = np.repeat(np.arange(pairs) * 2.0, 2)
+    pos[1::2, 0] = 1.0
+    th = values(rng, pairs, lo, hi, zeros=0.02)
+    th[::7] = np.round(th[::7] / np.pi) * np.pi  # near the sine's zeros
+    amp = np.where(rng.random(pairs) < 0.2, rng.uniform(4.0, 9.0, pairs), rng.uniform(-0.3, 0.3, pairs))
+    sc = wl.empty_scene(1e-4, (0.0, 0.0, 0.0))
+    sc.update(pos=pos, vel=np.zeros((n, 3)), m=np.ones(n), left=np.arange(0, n, 2, dtype=np.int32),
+              right=np.arange(1, n, 2, dtype=np.int32), k=np.ones(pairs), rest=np.ones(pairs), damping=np.zeros(pairs),
+              type=rng.integers(2, 4, pairs).astype(np.int32), omega=np.zeros(pairs), amp=amp, phase=th)
+    s = wl.make_sim(sc, tg.FP64, 64)
+    s.step(1)
+    got = s.get_state(acc=True)["acc"][1::2, 0]
+    want = (1.0 + np.where(sc["type"] == 2, -amp, amp) * np.sin(th)) - 1.0
+    scale = np.maximum(1.0, np.abs(1.0 + want))
+    assert np.all(np.abs(got - want) <= (5 * np.abs(amp) + 2 * scale) * 2.0 ** -52)

@@ -1,6 +1,7 @@
-// fp64_alu.cuh -- FP64 square root, division and product on the integer
-// units, correctly rounded (round to nearest even): the bits of the IEEE
-// operation, which is what the FP64 form's parity with the CPU oracle needs.
+// fp64_alu.cuh -- FP64 square root, division, product and sine on the integer
+// units.  The first three are correctly rounded (round to nearest even): the
+// bits of the IEEE operation, which is what the FP64 form's parity with the
+// CPU oracle needs.
 //
 // Why: GB300 executes 1.6 FP64 operations per SM and clock (measured, any of
 // add, multiply, fma, compare or conversion: a warp instruction takes 20
@@ -289,6 +290,75 @@ TG_HD Alu alu_sqrt(const Alu &n, AluDivisor &d) {
     const int es = h - 26 + 1075;
     d = AluDivisor{S, y63 + (uint64_t)(int64_t)corr, es, 0};
     return Alu{S, es, 0};
+}
+
+// sin(x) for 2^-24 <= |x| < 2^30 (alu_sin_range): the turn fraction x / 2 pi
+// modulo 1 from the exact product of the significand with 96 bits of 1/2 pi,
+// folded to a quarter turn X and summed as X (d0 - t (d1 - t (d2 - ...))),
+// t = X^2, d_k = (pi/2)^(2k+1) / (2k+1)!: the Taylor series of the sine, cut
+// where its terms are below 2^-67.  Absolute error below 2^-59 before the
+// one rounding to 53 bits.
+TG_HD bool alu_sin_range(double x) {
+    const uint32_t e = (alu_hi(alu_bits(x)) >> 20) & 0x7ffu;
+    return e - (1023u - 24u) < 54u;
+}
+
+TG_HD Alu alu_sin(double x) {
+    const uint64_t b = alu_bits(x);
+    const uint32_t bh = alu_hi(b);
+    const uint32_t mh = (bh & 0xfffffu) | 0x100000u, ml = alu_lo(b);
+    const uint32_t e = (bh >> 20) & 0x7ffu;
+    // |x| / 2 pi = (m K) 2^(e - 1075 - 96); words w4..w1 of m K (w0 dropped)
+    constexpr uint32_t k2 = 0x28be60dbu, k1 = 0x9391054au, k0 = 0x7f09d5f4u;
+    uint64_t lo = alu_mad(ml, k1, alu_mulhi(ml, k0));
+    const uint64_t hi = alu_mad(ml, k2, alu_hi(lo));
+    uint64_t r = alu_mad(mh, k0, alu_lo(lo));
+    const uint32_t w1 = alu_lo(r);
+    r = alu_mad(mh, k1, (uint64_t)alu_lo(hi) + alu_hi(r));
+    const uint32_t w2 = alu_lo(r);
+    r = alu_mad(mh, k2, (uint64_t)alu_hi(hi) + alu_hi(r));
+    const uint32_t w3 = alu_lo(r), w4 = alu_hi(r);
+    // the 64 bits below the binary point: bit 1107 - e - 32 (of w1's lowest
+    // upwards) in [22, 75]
+    const uint32_t at = 1075u - e;
+    const uint32_t v0 = at >= 64 ? w3 : (at >= 32 ? w2 : w1), v1 = at >= 64 ? w4 : (at >= 32 ? w3 : w2),
+                   v2 = at >= 64 ? 0u : (at >= 32 ? w4 : w3);
+    uint32_t f0 = alu_shr(v0, v1, at & 31), f1 = alu_shr(v1, v2, at & 31);
+    // fold: turns in [1/4, 3/4) are mirrored; then |turns| <= 1/4
+    const bool mirror = ((f1 + 0x40000000u) & 0x80000000u) != 0;
+    uint64_t f = alu_join(f1, f0);
+    if (mirror) f = 0x8000000000000000ull - f;
+    const uint32_t neg = alu_hi(f) & 0x80000000u;
+    if (neg) f = 0 - f;
+    // X and t in units of 2^-64, the terms from k = 6 down in 2^-63
+    const uint64_t X = f >= 0x4000000000000000ull ? ~0ull : f << 2;
+    const uint64_t T = alu_mulhi64(X, X);
+    const uint32_t t = alu_hi(T);
+    uint32_t q = 0x251u - alu_mulhi(t, 3u);  // units of 2^-61, from k = 10
+    q = 0x18a40u - alu_mulhi(t, q);
+    q = 0xd57619u - alu_mulhi(t, q);
+    q = 0x5beb6e7cu - alu_mulhi(t, q);
+    uint64_t p = 0x7a3d0d3406ull - ((uint64_t)alu_mulhi(t, q) << 2);
+    p = 0x1e3074fde887ull - alu_mulhi64(T, p);
+    p = 0x541e0d21fb9e0ull - alu_mulhi64(T, p);
+    p = 0x9969667315ec2eull - alu_mulhi64(T, p);
+    p = 0xa335e33bad570e9ull - alu_mulhi64(T, p);
+    p = 0x52aef39896f94afbull - alu_mulhi64(T, p);
+    p = 0xc90fdaa22168c235ull - alu_mulhi64(T, p);
+    uint64_t s = alu_mulhi64(X, p);
+    // to 53 bits, round to nearest
+    Alu a;
+    a.sign = (bh & 0x80000000u) ^ neg;
+#ifdef __CUDA_ARCH__
+    const int z = __clzll((long long)s);
+#else
+    const int z = s ? __builtin_clzll(s) : 64;
+#endif
+    s <<= z & 63;
+    a.m = (s + 0x400u) >> 11;
+    if (s > ~0ull - 0x400u) a.m = 1ull << 53;
+    a.e = s ? 1023 - z : kAluZero;
+    return a;
 }
 
 }  // namespace tg

@@ -119,6 +119,28 @@ __device__ __noinline__ F3<P_FP64> spring_force_f64_wide(int sa, int sb, double 
     return F3<P_FP64>{f0, f1, f2};
 }
 
+// FP64 rest length of an actuated spring, rest (1 -+ amp sin th), with the
+// FP64 instructions alone.
+__device__ __noinline__ double actuated_rest_f64_wide(double rest, double amp, double th, uint32_t type) {
+    const double sn = amp * sin(th);
+    return rest * (type == 2 ? 1.0 - sn : 1.0 + sn);
+}
+
+// The same with the sine and the products on the integer units, for angles
+// in alu_sin's range and amplitudes below 4: the sine is then within 0.51 of
+// a unit in the last place where it is above 1/2 and within 2^-59 elsewhere,
+// which 1 -+ amp sin th rounds away.
+__device__ __forceinline__ double actuated_rest_f64(double rest, double amp, double th, uint32_t type) {
+    bool bad = !alu_sin_range(th);
+    const Alu am = alu_unpack(amp, bad);
+    bad |= am.e > 1024;
+    Alu sn = alu_sin(th);
+    alu_carry(sn);
+    const double q = alu_pack(alu_mul(am, sn));
+    const double r = alu_pack(alu_mul(alu_unpack(rest, bad), alu_unpack(type == 2 ? 1.0 - q : 1.0 + q, bad)));
+    return bad ? actuated_rest_f64_wide(rest, amp, th, type) : r;
+}
+
 // FP64 force: the reference's operations in the reference's order, the
 // additions on the FP64 pipe, the square root, divisions and products on the
 // integer units (fp64_alu.cuh: the same bits).
@@ -167,12 +189,9 @@ __device__ __forceinline__ F3<PREC> spring_force(int sa, int sb, uint32_t type, 
     if constexpr (PREC == P_FP64) {
         double rs = rest;  // rest * scale; a scale of 1 changes nothing
         if (actuated) {
-            const double2 q01 = act.lo;
-            const double2 q23 = act.hi;
-            double th = q01.x * t.T;
-            th = th + q23.x;
-            const double sn = q01.y * sin(th);
-            rs = rest * (type == 2 ? 1.0 - sn : 1.0 + sn);
+            double th = act.lo.x * t.T;
+            th = th + act.hi.x;
+            rs = actuated_rest_f64(rest, act.lo.y, th, type);
         }
         return spring_force_f64(sa, sb, k, rs, damping, st);
     } else {
