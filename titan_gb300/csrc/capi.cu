@@ -743,10 +743,17 @@ int build_device(titan_gb300_sim *s) {
     }
     s->plan_tile = in.tile_cap;
     const tg::Plan &P = s->plan;
-    // threads per CTA of the per-tile forms: one per tile mass (two in FP64)
-    s->threads = s->threads_req > 0
-                     ? s->threads_req
-                     : std::max(128, std::min(512, ((P.max_nm + 31) / 32) * 32 * (s->prec == P_FP64 ? 2 : 1)));
+    // threads per CTA of the per-tile forms: one per tile mass, in FP64 two,
+    // and there at least 256 while every tile gets a CTA at once (two of 256
+    // threads fit one SM; tiles of 32 masses: 11.3 us per step of the 5^3
+    // lattice against 12.1 with 128, 16.1 against 18.4 of a 20^3 one; with
+    // more tiles the second wave costs more: 30 against 25 us at 385)
+    int sms_dev = 0;
+    CK(cudaDeviceGetAttribute(&sms_dev, cudaDevAttrMultiProcessorCount, s->device), "device");
+    const int min_threads = s->prec == P_FP64 && P.ntiles <= 2 * sms_dev ? 256 : 128;
+    s->threads = s->threads_req > 0 ? s->threads_req
+                                    : std::max(min_threads, std::min(512, ((P.max_nm + 31) / 32) * 32 *
+                                                                              (s->prec == P_FP64 ? 2 : 1)));
     s->npad = ((s->n + 127) / 128) * 128;
     const int64_t np = s->npad;
     auto &a = s->args;

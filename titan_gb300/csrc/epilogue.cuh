@@ -34,9 +34,10 @@ __device__ __forceinline__ void integrate(const StepArgs &a, const TileInfo &ti,
                                           const DevParams *prm) {
     if constexpr (PREC == P_FP64) {
         double Fd[3] = {F0, F1, F2};
-        Fd[0] = Fd[0] + prm->g[0] * m;
-        Fd[1] = Fd[1] + prm->g[1] * m;
-        Fd[2] = Fd[2] + prm->g[2] * m;
+        const D3 gm = mul3_alu(prm->g, m);
+        Fd[0] = Fd[0] + gm.x;
+        Fd[1] = Fd[1] + gm.y;
+        Fd[2] = Fd[2] + gm.z;
         if (fl & MF_EXT) {
             const double *ext = reinterpret_cast<const double *>(a.ext);
             Fd[0] = Fd[0] + ext[g];
@@ -63,7 +64,8 @@ __device__ __forceinline__ void integrate(const StepArgs &a, const TileInfo &ti,
             }
         }
         const double dt = prm->dt;
-        double acc[3] = {Fd[0] / m, Fd[1] / m, Fd[2] / m};
+        const D3 fm = div3_alu(Fd, m);
+        const double acc[3] = {fm.x, fm.y, fm.z};
         double *ac = reinterpret_cast<double *>(a.acc);
         const int integ = INTEG >= 0 ? INTEG : prm->integrator;
         if (integ == INTEG_VERLET) {  // src/sim.cu:1155-1159; acc is state
@@ -89,11 +91,14 @@ __device__ __forceinline__ void integrate(const StepArgs &a, const TileInfo &ti,
                 for (int c = 0; c < 3; c++) s.v[c] = b.v[c] + acc[c] * dt;
             }
         } else {  // symplectic Euler, src/sim.cu:1161-1166
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                s.v[c] = s.v[c] + acc[c] * dt;
-                s.x[c] = s.x[c] + s.v[c] * dt;
-            }
+            const D3 dv = mul3_alu(acc, dt);
+            s.v[0] = s.v[0] + dv.x;
+            s.v[1] = s.v[1] + dv.y;
+            s.v[2] = s.v[2] + dv.z;
+            const D3 dx = mul3_alu(s.v, dt);
+            s.x[0] = s.x[0] + dx.x;
+            s.x[1] = s.x[1] + dx.y;
+            s.x[2] = s.x[2] + dx.z;
         }
         store_state<PREC>(out, gs, s);
         if (write_acc) {

@@ -18,20 +18,19 @@
 // exponent.  The square root and the quotient are integers Q with a known
 // exact remainder condition: an estimate from a reciprocal (square root)
 // good to about 2^-59 -- a 22-bit FP32 hardware estimate improved by one
-// third-order step, y (1 + e/2 + 3 e^2/8) with e = 1 - n y^2, or y (1 + e +
-// e^2) with e = 1 - n y (over all FP32 significands |e| < 2^-20.8 and
-// 2^-21.8 on the GPU, so what the step leaves out is below 2^-64) -- gives Q to within a little more than half a unit,
+// third-order step, y (1 + e/2 + 3 e^2/8) with e = 1 - n y^2, or y (1 - f +
+// f^2) with f = n y - 1 (over all FP32 significands |e| < 2^-20.8 and
+// |f| < 2^-21.8 on the GPU, so what the step leaves out is below 2^-64) -- gives Q to within a little more than half a unit,
 // biased down, and the exact remainder modulo 2^64 (it is far smaller than
 // 2^63 in magnitude) says whether the next integer is nearer.  Neither a
 // quotient nor a square root of 53-bit operands can lie half-way between two
 // 53-bit numbers, so no tie arises; a product's does, and is rounded from
 // its exact 106 bits.
 //
-// Range: operands are normal with exponents in [2^-250, 2^250], or zero (an
-// exponent of kAluZero, carried through products and quotients: a result
-// with a negative exponent is a zero).  alu_unpack reports anything else
-// (subnormals, infinities, NaN, huge and tiny values) in `bad`; the caller
-// then uses the FP64 instructions.
+// Range: operands are zero or normal with exponents in [-255, 256].  alu_unpack
+// collects in `bad` what is outside (subnormals, infinities, NaN, huge and
+// tiny values); the caller then uses the FP64 instructions.  A zero carries
+// an exponent far below any other through products and quotients.
 //
 // The host compiles the same functions (with its own initial estimates), so
 // that they are also tested on the CPU.
@@ -49,15 +48,17 @@
 
 namespace tg {
 
-constexpr int kAluZero = -100000;  // exponent of a zero
-constexpr int kAluLo = 1023 - 250, kAluHi = 1023 + 250;
-
-// value = (-1)^sign * m * 2^(e - 1075), m in [2^52, 2^53); e <= 0: zero
+// value = (-1)^s m 2^(e - 1075), m in [2^52, 2^53) (functions say where 2^53
+// may be returned and is taken).  se holds the sign in bit 31 and e + kAluBias
+// below it, so that one addition gives a product's sign and exponent; e < 0,
+// bit 20 clear, is a zero.
 struct Alu {
     uint64_t m;
-    int e;
-    uint32_t sign;  // 0 or 0x80000000
+    uint32_t se;
 };
+constexpr uint32_t kAluBias = 0x100000u, kAluZeroDrop = 0x8000u;
+// nonzero operands in range leave these bits of `bad` clear
+constexpr uint32_t kAluBadBits = 0x60000000u;
 
 TG_HD uint64_t alu_bits(double x) {
 #ifdef __CUDA_ARCH__
@@ -143,51 +144,54 @@ TG_HD float alu_float(uint32_t b) {
 #endif
 }
 
-TG_HD Alu alu_unpack(double x, bool &bad) {
+TG_HD Alu alu_unpack(double x, uint32_t &bad) {
     const uint64_t b = alu_bits(x);
     const uint32_t h = alu_hi(b);
     Alu a;
-    a.sign = h & 0x80000000u;
-    a.e = (int)((h >> 20) & 0x7ffu);
     a.m = alu_join((h & 0xfffffu) | 0x100000u, alu_lo(b));
-    const bool in = (uint32_t)(a.e - kAluLo) <= (uint32_t)(kAluHi - kAluLo);
-    const bool zero = ((h << 1) | alu_lo(b)) == 0;
-    bad |= !(in || zero);
-    if (zero) a.e = kAluZero;
+    a.se = ((uint32_t)((int32_t)h >> 20) & 0x800007ffu) | kAluBias;
+    if (((h & 0x7fffffffu) | alu_lo(b)) == 0)
+        a.se -= kAluZeroDrop;
+    else
+        bad |= (h + 0x10000000u) ^ 0x40000000u;  // exponent fields 768..1279: bits 30, 29 = 1, 0
     return a;
 }
+TG_HD bool alu_bad(uint32_t bad) { return (bad & kAluBadBits) != 0; }
+TG_HD bool alu_nonzero(const Alu &a) { return (a.se & kAluBias) != 0; }
 
+// m may be 2^53
 TG_HD double alu_pack(const Alu &a) {
-    // m's top bit adds one to the exponent field
-    const uint32_t h = alu_hi(a.m) + ((uint32_t)(a.e - 1) << 20);
-    const bool nz = a.e > 0;
-    return alu_double(alu_join((nz ? h : 0u) | a.sign, nz ? alu_lo(a.m) : 0u));
+    const uint32_t h = alu_hi(a.m) + (a.se << 20) - 0x100000u;  // m's top bit adds one to the exponent field
+    const bool nz = alu_nonzero(a);
+    return alu_double(alu_join(((nz ? h : 0u) & 0x7fffffffu) | (a.se & 0x80000000u), nz ? alu_lo(a.m) : 0u));
 }
 
 // m = 2^53 (a significand rounded up over the top) becomes 2^52
 TG_HD void alu_carry(Alu &a) {
     const uint32_t c = alu_hi(a.m) >> 21;
-    a.m >>= c;
-    a.e += (int)c;
+    a.m = alu_join(alu_hi(a.m) >> c, alu_lo(a.m));  // the low bits of 2^53 are zero
+    a.se += c;
 }
 
-// The product's 106 bits hi : w rounded to 53: hi in [2^52, 2^54), w the 32
-// bits below it with a sticky lowest bit.
-TG_HD Alu alu_round(uint64_t hi, uint32_t w, int e, uint32_t sign) {
+// The 106-bit product hi : w (hi in [2^52, 2^54), w the 32 bits below it with
+// a sticky lowest bit) rounded to 53 bits.
+TG_HD Alu alu_round(uint64_t hi, uint32_t w, uint32_t se) {
     const uint32_t s = alu_hi(hi) >> 21;  // 1: hi has 54 bits
-    const uint32_t h = alu_hi(hi) >> s, l = alu_shr(alu_lo(hi), alu_hi(hi), s);
+    uint32_t h = alu_hi(hi) >> s, l = alu_shr(alu_lo(hi), alu_hi(hi), s);
     // below the half-way bit: the sticky bit, and l's lowest (half-way cases
     // go to the even neighbour)
     w = alu_shr(w, alu_lo(hi), s) | ((w | l) & 1u);
-    Alu r;
-    r.m = alu_join(h, l) + (w > 0x80000000u ? 1u : 0u);
-    r.e = e + (int)s;
-    r.sign = sign;
-    return r;
+#ifdef __CUDA_ARCH__
+    // w above one half carries into the significand
+    asm("add.cc.u32 %2, %2, 0x7fffffff;\n addc.cc.u32 %0, %0, 0;\n addc.u32 %1, %1, 0;" : "+r"(l), "+r"(h), "+r"(w));
+    return Alu{alu_join(h, l), se + s};
+#else
+    return Alu{alu_join(h, l) + (w > 0x80000000u ? 1u : 0u), se + s};
+#endif
 }
+TG_HD uint32_t alu_sticky(uint32_t x) { return x < 1u ? x : 1u; }
 
-// a * b; the result's m may be 2^53 (alu_pack takes that; alu_carry for
-// further use as an operand)
+// a * b; a's m may be 2^53, and the result's
 TG_HD Alu alu_mul(const Alu &a, const Alu &b) {
     const uint64_t x = a.m << 1, y = b.m << 11;
     const uint32_t xl = alu_lo(x), xh = alu_hi(x), yl = alu_lo(y), yh = alu_hi(y);
@@ -195,8 +199,7 @@ TG_HD Alu alu_mul(const Alu &a, const Alu &b) {
     const uint64_t t = alu_mad(xl, yh, alu_hi(p));
     const uint64_t u = alu_mad(xh, yl, alu_lo(t));
     const uint64_t hi = alu_mad(xh, yh, (uint64_t)alu_hi(t)) + alu_hi(u);
-    const uint32_t w = alu_lo(u) | (alu_lo(p) != 0 ? 1u : 0u);
-    return alu_round(hi, w, a.e + b.e - 1023, a.sign ^ b.sign);
+    return alu_round(hi, alu_lo(u) | alu_sticky(alu_lo(p)), a.se + b.se - (1023u + kAluBias));
 }
 
 TG_HD Alu alu_square(const Alu &a) {
@@ -205,30 +208,27 @@ TG_HD Alu alu_square(const Alu &a) {
     const uint64_t p = alu_mad(xl, xl, 0);
     const uint64_t t = alu_mad(xl, xh << 1, alu_hi(p));  // xh < 2^27
     const uint64_t hi = alu_mad(xh, xh, (uint64_t)alu_hi(t));
-    const uint32_t w = alu_lo(t) | (alu_lo(p) != 0 ? 1u : 0u);
-    return alu_round(hi, w, 2 * a.e - 1023, 0);
+    return alu_round(hi, alu_lo(t) | alu_sticky(alu_lo(p)), a.se + a.se - (1023u + kAluBias));
 }
 
-// A divisor: significand, exponent and reciprocal, r = 2^115 / m (2^62 <= r
-// <= 2^63), relative error below 2^-58.5.
+// A divisor: significand, sign and exponent, and reciprocal r = 2^115 / m
+// (2^62 <= r <= 2^63), relative error below 2^-58.5.
 struct AluDivisor {
     uint64_t m, r;
-    int e;
-    uint32_t sign;
+    uint32_t se;
 };
 
-// a / d; the result's m may be 2^53
+// a / d
 TG_HD Alu alu_div(const Alu &a, const AluDivisor &d) {
-    const uint64_t t = alu_mulhi64(a.m << 11, d.r);  // (a.m / d.m) 2^62, within 24
-    const uint32_t s = (alu_hi(t) >> 30) ^ 1u;       // 0: a.m >= d.m, 53 bits are t >> 10; 1: t >> 9
-    // nearest integer from below: 64 units of 2^9 or 2^10 short of half
-    uint64_t q = (t + ((512u >> s) - 64u)) >> (10 - s);
-    // exact remainder a.m 2^(52+s) - q d.m
-    const uint64_t num = alu_join(alu_lo(a.m) << (20 + s), 0);
-    const uint64_t rem = num - alu_mullo64(q, d.m);
-    const uint64_t x = d.m - (rem << 1);
-    q += alu_hi(x) >> 31;
-    return Alu{q, a.e - d.e + 1023 - (int)s, a.sign ^ d.sign};
+    const bool lt = a.m < d.m;
+    const uint64_t x = lt ? a.m << 1 : a.m;        // x / d.m in [1, 2)
+    const uint64_t t = alu_mulhi64(x << 10, d.r);  // (x / d.m) 2^61, within 24
+    // nearest integer from below: 64 units of 2^-9 short of half
+    uint64_t q = (t + (256u - 64u)) >> 9;
+    // exact remainder x 2^52 - q d.m
+    const uint64_t rem = alu_join(alu_lo(x) << 20, 0) - alu_mullo64(q, d.m);
+    q += alu_hi(d.m - (rem << 1)) >> 31;
+    return Alu{q, a.se - d.se + (1023u + kAluBias) - (lt ? 1u : 0u)};
 }
 
 // |x| as a divisor from its unpacked form (not zero)
@@ -236,27 +236,24 @@ TG_HD AluDivisor alu_divisor(const Alu &x) {
     // y23 2^-23 = 1/v, v = m 2^-52 in [1, 2)
     const float v = alu_float(0x3f800000u | alu_lo(x.m >> 29));  // m's bit 52 lands on exponent bit 0, set already
     const uint32_t y = alu_float_bits(alu_rcp_estimate(v) + 1.0f) - 0x3f800000u;
-    // e = 1 - v y: m y in units of 2^-75 -> keep 2^-64 (modulo 1: |e| < 2^-19)
+    // f = v y - 1: m y in units of 2^-75 -> keep 2^-64 (modulo 1: |f| < 2^-21)
     const uint64_t lo = (uint64_t)alu_lo(x.m) * y;
     const uint64_t prod_hi = alu_mad(alu_hi(x.m), y, lo >> 32);  // units of 2^-43
-    const uint64_t e64 = 0 - ((prod_hi << 21) | (alu_lo(lo) >> 11));
-    const int64_t e = (int64_t)e64;
-    const int32_t et = (int32_t)(e >> 16);                          // units of 2^-48
-    const uint32_t et_abs = (uint32_t)(et < 0 ? -et : et);
-    const uint32_t e2 = alu_mulhi(et_abs, et_abs);                  // e^2, units of 2^-64
-    const uint64_t c = e64 + e2;                                    // e + e^2, 2^-64
-    // r = 2^63 y23 2^-23 (1 + c)
-    const uint64_t yc = ((uint64_t)y * alu_lo(c)) >> 24;            // 2^63 2^-23 2^-64 = 2^-24
-    const int64_t yh = (int64_t)(int32_t)alu_hi(c) * (int32_t)y;    // times 2^32: << 8
-    return AluDivisor{x.m, ((uint64_t)y << 40) + (uint64_t)(yh * 256) + yc, x.e, x.sign};
+    const uint64_t f64 = (prod_hi << 21) | (alu_lo(lo) >> 11);
+    const int32_t ft = (int32_t)((int64_t)f64 >> 16);            // units of 2^-48
+    const uint32_t ft_abs = (uint32_t)(ft < 0 ? -ft : ft);
+    const uint64_t c = f64 - alu_mulhi(ft_abs, ft_abs);          // f - f^2, units of 2^-64
+    // r = 2^63 y23 2^-23 (1 - c)
+    const uint64_t yc = ((uint64_t)y * alu_lo(c)) >> 24;         // 2^63 2^-23 2^-64 = 2^-24
+    const int64_t yh = (int64_t)(int32_t)alu_hi(c) * (int32_t)y; // times 2^32: << 8
+    return AluDivisor{x.m, ((uint64_t)y << 40) - (uint64_t)(yh * 256) - yc, x.se};
 }
 
 // sqrt of the positive number n, and the result as a divisor
 TG_HD Alu alu_sqrt(const Alu &n, AluDivisor &d) {
     // n = N 2^(2h), N in [2^52, 2^54)
-    const uint32_t odd = (uint32_t)(n.e - 1075) & 1u;
-    const uint64_t N = n.m << odd;
-    const int h = (n.e - 1075 - (int)odd) >> 1;
+    const uint32_t odd = (n.se & 1u) ^ 1u;  // of e - 1075
+    const uint64_t N = odd ? n.m << 1 : n.m;
     // y 2^-23 = 1/sqrt(N 2^-52)
     const float v = alu_float((0x3f800000u + (odd << 23)) | (alu_lo(n.m >> 29) & 0x7fffffu));
     const uint32_t y = alu_float_bits(alu_rsqrt_estimate(v) + 1.0f) - 0x3f800000u;
@@ -287,9 +284,10 @@ TG_HD Alu alu_sqrt(const Alu &n, AluDivisor &d) {
     const uint32_t y16 = alu_hi(y63) >> 15;
     const uint32_t y3 = (((y16 * y16) >> 16) * y16) >> 16;  // y16 = 2^16 where y = 1
     const int32_t corr = ((int32_t)alu_hi(rho) * (int32_t)(y3 >> 7)) >> 19;
-    const int es = h - 26 + 1075;
-    d = AluDivisor{S, y63 + (uint64_t)(int64_t)corr, es, 0};
-    return Alu{S, es, 0};
+    // e of the root: (e - 1075 - odd) / 2 - 26 + 1075
+    const uint32_t se = ((n.se - kAluBias + 1023u - odd) >> 1) + kAluBias;
+    d = AluDivisor{S, y63 + (uint64_t)(int64_t)corr, se};
+    return Alu{S, se};
 }
 
 // sin(x) for 2^-24 <= |x| < 2^30 (alu_sin_range): the turn fraction x / 2 pi
@@ -348,7 +346,6 @@ TG_HD Alu alu_sin(double x) {
     uint64_t s = alu_mulhi64(X, p);
     // to 53 bits, round to nearest
     Alu a;
-    a.sign = (bh & 0x80000000u) ^ neg;
 #ifdef __CUDA_ARCH__
     const int z = __clzll((long long)s);
 #else
@@ -357,7 +354,7 @@ TG_HD Alu alu_sin(double x) {
     s <<= z & 63;
     a.m = (s + 0x400u) >> 11;
     if (s > ~0ull - 0x400u) a.m = 1ull << 53;
-    a.e = s ? 1023 - z : kAluZero;
+    a.se = ((bh & 0x80000000u) ^ neg) | (kAluBias + (s ? 1023u - (uint32_t)z : 0u - kAluZeroDrop));
     return a;
 }
 

@@ -123,7 +123,7 @@ __device__ __forceinline__ void tile_step(const StepArgs &a, const TileInfo &ti,
         }
     }
     // the first incidence words of this thread's mass
-    if (i_own < ti.nm && d_own != 255) {
+    if (PREC != P_FP64 && i_own < ti.nm && d_own != 255) {
         const uint2 *ip = reinterpret_cast<const uint2 *>(a.inc + woff_own) + (i_own & 31);
         const uint32_t nw = (d_own + 3) >> 2;
 #pragma unroll
@@ -167,6 +167,39 @@ __device__ __forceinline__ void tile_step(const StepArgs &a, const TileInfo &ti,
         __syncthreads();
     }
 
+    // ---- C1 (FP64): the three components of a mass's sum in different warps,
+    // where the CTA has a thread for each.  The sums are a chain of FP64
+    // additions, 64 cycles each on one SM sub-partition, and a 32-mass tile
+    // would leave three of the four idle (20^3 lattice, 256 threads: 17.3 ->
+    // 16.2 us per step).  Large tiles keep the sub-partitions busy with whole
+    // masses, and reading the incidence words three times costs them 4 %.
+    const bool split = PREC == P_FP64 && 2 * ti.nh >= ti.nm && 3 * ((ti.nm + 31) & ~31) <= (int)blockDim.x;
+    double *sF = reinterpret_cast<double *>(st + (int64_t)ti.nm * kRec);  // over the halo's records: 3 * nm
+    if (split) {
+        const int nmp = (ti.nm + 31) & ~31;
+        const int c = threadIdx.x >= 2 * nmp ? 2 : (threadIdx.x >= nmp ? 1 : 0), i = threadIdx.x - c * nmp;
+        if (i < ti.nm) {
+            const uint32_t d = __ldg(a.deg + ti.mass_off + i);
+            double F = 0;
+            if (d != 255) {
+                const uint2 *ip =
+                    reinterpret_cast<const uint2 *>(a.inc + __ldg(a.warp_inc_off + ti.warp_off + (i >> 5))) + (i & 31);
+                const uint32_t nw = (d + 3) >> 2;
+                for (uint32_t w0 = 0; w0 < nw; w0 += kBatchC) {
+                    uint2 cw[kBatchC];
+#pragma unroll
+                    for (int k = 0; k < kBatchC; k++)
+                        if (w0 + k < nw) cw[k] = __ldg(ip + 32 * (w0 + k));
+#pragma unroll
+                    for (int k = 0; k < kBatchC; k++)
+                        if (w0 + k < nw) F = gather_word_component(slots, cw[k], c, F);
+                }
+            }
+            sF[c * ti.nm + i] = F;
+        }
+        __syncthreads();
+    }
+
     // ---- C: per-mass gather, constraints, integration ----------------------
     for (int i = threadIdx.x; i < ti.nm; i += blockDim.x) {
         const int64_t g = (int64_t)ti.mass_off + i;
@@ -182,12 +215,16 @@ __device__ __forceinline__ void tile_step(const StepArgs &a, const TileInfo &ti,
             F0 = F0 + sH[h];
             F1 = F1 + sH[ti.nheavy + h];
             F2 = F2 + sH[2 * ti.nheavy + h];
+        } else if (split) {
+            F0 = (R)sF[i];
+            F1 = (R)sF[ti.nm + i];
+            F2 = (R)sF[2 * ti.nm + i];
         } else if (d > 0) {
             const uint32_t woff = own ? woff_own : __ldg(a.warp_inc_off + ti.warp_off + (i >> 5));
             const uint2 *ip = reinterpret_cast<const uint2 *>(a.inc + woff) + (i & 31);
             const uint32_t nw = (d + 3) >> 2;
             uint32_t w0 = 0;
-            if (own) {
+            if (PREC != P_FP64 && own) {
 #pragma unroll
                 for (int w = 0; w < kPrefetchW; w++)
                     if ((uint32_t)w < nw) gather_word_padded<PREC>(slots, cw_own[w], F0, F1, F2);

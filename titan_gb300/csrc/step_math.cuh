@@ -4,6 +4,7 @@
 #pragma once
 
 #include "engine.h"
+#include "fp64_alu.cuh"
 
 namespace tg {
 namespace {
@@ -18,10 +19,58 @@ __device__ __forceinline__ double dot3(const double *a, const double *b) {
     return (a[0] * b[0] + a[1] * b[1]) + a[2] * b[2];
 }
 
+// The same with the products and the square root on the integer units
+// (fp64_alu.cuh: the same bits), and a vector times or divided by a number;
+// the _wide forms serve operands outside the integer path's range and are
+// kept out of line.  The epilogue then has 19 FP64 instructions per mass
+// where it had about 92 (a plane, a ball, Euler).
+struct D3 {
+    double x, y, z;
+};
+__device__ __noinline__ double dot3_wide(double a0, double a1, double a2, double b0, double b1, double b2) {
+    return (a0 * b0 + a1 * b1) + a2 * b2;
+}
+__device__ __noinline__ double nrm3_wide(double a, double b, double c) { return nrm3(a, b, c); }
+__device__ __noinline__ D3 mul3_wide(double a0, double a1, double a2, double b) { return D3{a0 * b, a1 * b, a2 * b}; }
+__device__ __noinline__ D3 div3_wide(double a0, double a1, double a2, double b) { return D3{a0 / b, a1 / b, a2 / b}; }
+
+__device__ __forceinline__ double dot3_alu(const double *a, const double *b) {
+    uint32_t bad = 0;
+    double p[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) p[c] = alu_pack(alu_mul(alu_unpack(a[c], bad), alu_unpack(b[c], bad)));
+    if (alu_bad(bad)) return dot3_wide(a[0], a[1], a[2], b[0], b[1], b[2]);
+    return (p[0] + p[1]) + p[2];
+}
+__device__ __forceinline__ double nrm3_alu(double a, double b, double c) {
+    uint32_t bad = 0;
+    const double q0 = alu_pack(alu_square(alu_unpack(a, bad))), q1 = alu_pack(alu_square(alu_unpack(b, bad))),
+                 q2 = alu_pack(alu_square(alu_unpack(c, bad)));
+    const Alu n2 = alu_unpack((q0 + q1) + q2, bad);
+    if (alu_bad(bad) || !alu_nonzero(n2)) return nrm3_wide(a, b, c);
+    AluDivisor d;
+    return alu_pack(alu_sqrt(n2, d));
+}
+__device__ __forceinline__ D3 mul3_alu(const double *a, double b) {
+    uint32_t bad = 0;
+    const Alu y = alu_unpack(b, bad);
+    const D3 r = {alu_pack(alu_mul(alu_unpack(a[0], bad), y)), alu_pack(alu_mul(alu_unpack(a[1], bad), y)),
+                  alu_pack(alu_mul(alu_unpack(a[2], bad), y))};
+    return alu_bad(bad) ? mul3_wide(a[0], a[1], a[2], b) : r;
+}
+__device__ __forceinline__ D3 div3_alu(const double *a, double b) {
+    uint32_t bad = 0;
+    const Alu y = alu_unpack(b, bad);
+    const AluDivisor d = alu_divisor(y);
+    const D3 r = {alu_pack(alu_div(alu_unpack(a[0], bad), d)), alu_pack(alu_div(alu_unpack(a[1], bad), d)),
+                  alu_pack(alu_div(alu_unpack(a[2], bad), d))};
+    return alu_bad(bad) || !alu_nonzero(y) ? div3_wide(a[0], a[1], a[2], b) : r;
+}
+
 // src/object.cu:73-106
 __device__ __forceinline__ void plane_apply(const double *n, double off, double fk, double fs,
                                             const double *x, const double *v, double *F) {
-    double disp = dot3(x, n) - off;
+    double disp = dot3_alu(x, n) - off;
     if (!(disp < 0)) return;  // only zeros would be added otherwise
     double fdn = dot3(F, n);
     double fn[3] = {n[0] * fdn, n[1] * fdn, n[2] * fdn};
@@ -52,7 +101,7 @@ __device__ __forceinline__ void plane_apply(const double *n, double off, double 
 // src/object.cu:53-56
 __device__ __forceinline__ void ball_apply(const double *c, double r, const double *x, double *F) {
     double d[3] = {x[0] - c[0], x[1] - c[1], x[2] - c[2]};
-    double dist = nrm3(d[0], d[1], d[2]);
+    double dist = nrm3_alu(d[0], d[1], d[2]);
     if (dist <= r) {
         F[0] = F[0] + (kNormal * d[0]) / dist;
         F[1] = F[1] + (kNormal * d[1]) / dist;

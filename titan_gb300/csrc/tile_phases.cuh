@@ -131,14 +131,14 @@ __device__ __noinline__ double actuated_rest_f64_wide(double rest, double amp, d
 // a unit in the last place where it is above 1/2 and within 2^-59 elsewhere,
 // which 1 -+ amp sin th rounds away.
 __device__ __forceinline__ double actuated_rest_f64(double rest, double amp, double th, uint32_t type) {
-    bool bad = !alu_sin_range(th);
+    uint32_t bad = 0;
     const Alu am = alu_unpack(amp, bad);
-    bad |= am.e > 1024;
+    const bool in = alu_sin_range(th) && (am.se & 0x7ffu) <= 1024u;
     Alu sn = alu_sin(th);
     alu_carry(sn);
     const double q = alu_pack(alu_mul(am, sn));
     const double r = alu_pack(alu_mul(alu_unpack(rest, bad), alu_unpack(type == 2 ? 1.0 - q : 1.0 + q, bad)));
-    return bad ? actuated_rest_f64_wide(rest, amp, th, type) : r;
+    return !in || alu_bad(bad) ? actuated_rest_f64_wide(rest, amp, th, type) : r;
 }
 
 // FP64 force: the reference's operations in the reference's order, the
@@ -149,19 +149,15 @@ __device__ __forceinline__ F3<P_FP64> spring_force_f64(int sa, int sb, double k,
     const double2 *pa = reinterpret_cast<const double2 *>(st + (int64_t)sa * 48);
     const double2 *pb = reinterpret_cast<const double2 *>(st + (int64_t)sb * 48);
     const double2 a0 = pa[0], a1 = pa[1], b0 = pb[0], b1 = pb[1];
-    bool bad = false;
+    uint32_t bad = 0;
     const Alu d0 = alu_unpack(b0.x - a0.x, bad), d1 = alu_unpack(b0.y - a0.y, bad),
               d2 = alu_unpack(b1.x - a1.x, bad);
     const Alu n2 = alu_unpack((alu_pack(alu_square(d0)) + alu_pack(alu_square(d1))) + alu_pack(alu_square(d2)), bad);
-    bad |= n2.e <= 0;
     AluDivisor nd;
     const double nrm = alu_pack(alu_sqrt(n2, nd));
     Alu fs = alu_mul(alu_unpack(k, bad), alu_unpack(rs - nrm, bad));
     alu_carry(fs);
-    Alu u0 = alu_div(d0, nd), u1 = alu_div(d1, nd), u2 = alu_div(d2, nd);
-    alu_carry(u0);
-    alu_carry(u1);
-    alu_carry(u2);
+    const Alu u0 = alu_div(d0, nd), u1 = alu_div(d1, nd), u2 = alu_div(d2, nd);
     double f0 = alu_pack(alu_mul(u0, fs)), f1 = alu_pack(alu_mul(u1, fs)), f2 = alu_pack(alu_mul(u2, fs));
     if (damping != 0.0) {
         const double2 a2 = pa[2], b2 = pb[2];
@@ -174,7 +170,7 @@ __device__ __forceinline__ F3<P_FP64> spring_force_f64(int sa, int sb, double k,
         f1 = f1 + alu_pack(alu_mul(u1, dd));
         f2 = f2 + alu_pack(alu_mul(u2, dd));
     }
-    if (bad) return spring_force_f64_wide(sa, sb, k, rs, damping, st);
+    if (alu_bad(bad) || !alu_nonzero(n2)) return spring_force_f64_wide(sa, sb, k, rs, damping, st);
     return F3<P_FP64>{f0, f1, f2};
 }
 
@@ -303,6 +299,19 @@ __device__ __forceinline__ void gather_word_padded(const uint8_t *slots, uint2 c
             F2 = fmaf(sg, f.z, F2);
         }
     }
+}
+
+// One component (0, 1, 2) of the FP64 forces that a whole word's codes name,
+// added in the same order.
+__device__ __forceinline__ double gather_word_component(const uint8_t *slots, uint2 cw, int c, double F) {
+#pragma unroll
+    for (int h = 0; h < 4; h++) {
+        const uint32_t word = h < 2 ? cw.x : cw.y;
+        const uint32_t code = (h & 1) ? (word >> 16) : (word & 0xffffu);
+        const double f = *reinterpret_cast<const double *>(slots + (int64_t)(code & 0x7fff) * 32 + 8 * c);
+        F = F + __hiloint2double(__double2hiint(f) ^ (int)((code & 0x8000u) << 16), __double2loint(f));
+    }
+    return F;
 }
 
 // Warp-cooperative, fixed-order sum over a heavy mass's incidence list
