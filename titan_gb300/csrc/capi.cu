@@ -150,6 +150,12 @@ struct titan_gb300_sim {
     std::vector<tg::TileInfo> rtiles;
     int rt_threads = 0, rt_mpt = 0;
     size_t rt_smem = 0;
+    // all tiles at once (resident_grid.cu); the per-step kernels stay ready
+    // for single steps
+    bool use_grid = false;
+    tg::GridResArgs gargs{};
+    int grid_shape = 0;
+    size_t grid_smem = 0;
     // plan taken from another handle with the same topology (adopt_plan);
     // used by the first start() only
     bool plan_adopted = false;
@@ -464,6 +470,7 @@ constexpr int kPullDefaultTile = 224;
 // 0.134 for the pull form with 160-mass tiles and three teams)
 constexpr bool kPullAuto = false;
 constexpr int kHeavyThreshold = 96;
+constexpr int64_t kGridMinSteps = 2;
 
 // Whether the step will run the pull form: when requested (set_kernel 6).
 // (It needs a plan without heavy masses: it has no warp-cooperative sums.)
@@ -480,7 +487,95 @@ bool pull_wanted(const titan_gb300_sim *s) {
     return true;
 }
 
-tg::PlanInput plan_input(titan_gb300_sim *s, int tile_masses) {
+int sm_count(const titan_gb300_sim *s) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device) != cudaSuccess || sms <= 0) {
+        cudaGetLastError();
+        sms = 152;  // GB300
+    }
+    return sms;
+}
+
+// Whether nothing chose another form than the resident grid for calls of
+// several steps.
+bool grid_wanted(const titan_gb300_sim *s) {
+    return s->kernel_req == 0 && s->res_mode == -1 && s->threads_req == 0 && s->min_ctas_req == 0 &&
+           s->res_threads_req == 0;
+}
+
+// The resident grid's launch for these tiles (resident_grid.cu): every tile
+// gets a CTA at once, with the slab in shared memory if that fits.  Small
+// tiles get small CTAs, which leave the SMs to other handles' kernels: FP64
+// 256 threads up to 300 entries, else 512 (9^3: 7.4 us per step with either,
+// 8.3 with 128); the FP32 forms 128 up to 400 entries, else 256 (16^3: 2.85
+// us with 128, 3.1 with 256; 24 scenes of 27 to 60,000 masses in flight
+// together, 200 steps: 8.2 against 10.5 ms).  Returns false when the tiles do
+// not all fit.
+bool choose_grid(const titan_gb300_sim *s, const std::vector<tg::TileInfo> &tiles, int &shape, int &stage, size_t &bytes) {
+    size_t smem[2] = {0, 0};
+    int max_nm = 0, max_ne = 0;
+    for (const tg::TileInfo &ti : tiles) {
+        max_nm = std::max(max_nm, (int)ti.nm);
+        max_ne = std::max(max_ne, (int)ti.ne);
+        for (int st = 0; st < 2; st++) smem[st] = std::max(smem[st], tg::grid_resident_smem_bytes(s->prec, ti, st));
+    }
+    int first;
+    if (s->prec == P_FP64) first = max_ne <= 300 ? 1 : 0;
+    else first = max_ne <= 400 ? 2 : 1;
+    const int order[3][tg::kGridShapes] = {{0, 1, 2}, {1, 0, 2}, {2, 1, 0}};
+    for (const int sh : order[first]) {
+        shape = sh;
+        const int ctas = tg::grid_resident_ctas(shape);
+        if ((int64_t)tiles.size() > (int64_t)sm_count(s) * ctas || max_nm > tg::grid_resident_threads(shape))
+            continue;
+        for (stage = 1; stage >= 0; stage--)
+            if (smem[stage] <= 227 * 1024 && (smem[stage] + 1024) * ctas <= 228 * 1024) {
+                bytes = smem[stage];
+                return true;
+            }
+    }
+    return false;
+}
+
+// Tile size with which the resident grid has all tiles at once, 0 if none:
+// the smallest that leaves one tile per SM in FP64 (each SM's FP64 pipe and
+// issue slots bind, and one CTA then has 512 threads) and two in the FP32
+// forms, where two CTAs fill each other's waits.  Measured, us per step, in
+// FP64 at 1 and 2 tiles per SM: 24^3 18.0 and 19.0, 30^3 28.9 and 31.0; in
+// FP32C 16^3 3.48 and 3.15, 30^3 6.6 and 6.2 -- and with the per-step
+// kernels 22.4, 32.2, 4.1 and 7.9.  At least 8 masses per tile in FP64 (9^3:
+// 7.4 us per step against 8.0 with 16), 16 in the FP32 forms (2.7 against 2.5
+// with 8, but half the CTAs).  Bodies up to whole masses stay one tile.
+// Above 192 masses (FP64) or 208 (FP32C: 63,000 in all) per tile the SM's
+// shared memory is too small; FP64 batches of bodies then try two per SM.
+int grid_tile(const titan_gb300_sim *s, int whole) {
+    const int64_t sms = sm_count(s);
+    auto tiles_of = [&](int t) {
+        if (s->body_ptr.empty()) return s->n <= whole ? (int64_t)1 : (s->n + t - 1) / t;
+        int64_t k = 0;
+        for (size_t b = 0; b + 1 < s->body_ptr.size(); b++) {
+            const int64_t m = s->body_ptr[b + 1] - s->body_ptr[b];
+            k += m <= whole ? 1 : (m + t - 1) / t;
+        }
+        return k;
+    };
+    auto smallest = [&](int64_t most, int hi) {
+        if (tiles_of(hi) > most) return 0;
+        int lo = std::min(hi, s->prec == P_FP64 ? 8 : 16);
+        while (lo < hi) {
+            const int mid = (lo + hi) / 2;
+            if (tiles_of(mid) <= most) hi = mid;
+            else lo = mid + 1;
+        }
+        return hi;
+    };
+    if (s->prec != P_FP64) return smallest(2 * sms, kWsDefaultTile);
+    const int t = smallest(sms, 192);
+    return t ? t : smallest(2 * sms, 128);
+}
+
+// grid: tiles for the resident grid where grid_tile has a size
+tg::PlanInput plan_input(titan_gb300_sim *s, int tile_masses, bool grid = false) {
     tg::PlanInput in;
     in.n = s->n;
     in.pos = s->pos.data();
@@ -510,11 +605,7 @@ tg::PlanInput plan_input(titan_gb300_sim *s, int tile_masses) {
     if (tile_masses > 0) {
         in.tile_cap = tile_masses;
     } else {
-        int sms = 0;
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device) != cudaSuccess || sms <= 0) {
-            cudaGetLastError();
-            sms = 152;  // GB300
-        }
+        const int sms = sm_count(s);
         auto fit = [&](double per_sm, int lo, int hi) {
             const int64_t t = (int64_t)((double)s->n / (per_sm * sms)) / 32 * 32;
             return (int)std::max<int64_t>(lo, std::min<int64_t>(hi, t));
@@ -529,6 +620,10 @@ tg::PlanInput plan_input(titan_gb300_sim *s, int tile_masses) {
             in.whole_cap = kWsDefaultTile;
         } else {
             in.tile_cap = 256;
+        }
+        if (const int t = grid && grid_wanted(s) && !pull ? grid_tile(s, in.whole_cap) : 0) {
+            in.tile_cap = t;
+            in.tile_min = 8;
         }
     }
     in.heavy_threshold = kHeavyThreshold;
@@ -713,8 +808,17 @@ int setup_pull(titan_gb300_sim *s, std::vector<tg::TileInfo> &tiles_run) {
 // tile of the warp-specialised form (208 masses) gives way to 192 when two
 // stages of the planned tiles would not fit one SM's shared memory.
 std::string plan_scene(titan_gb300_sim *s, int tile_masses, tg::PlanInput &in) {
-    in = plan_input(s, tile_masses);
-    std::string why = tg::build_plan(in, s->plan);
+    s->plan_req = tile_masses;
+    in = plan_input(s, tile_masses, true);
+    std::string why;
+    if (in.tile_min < 32) {  // tiles for the resident grid, if it takes them (heavy masses may split tiles)
+        int shape, stage;
+        size_t bytes;
+        why = tg::build_plan(in, s->plan);
+        if (why.empty() && choose_grid(s, tile_infos(s->plan), shape, stage, bytes)) return why;
+        in = plan_input(s, tile_masses);
+    }
+    why = tg::build_plan(in, s->plan);
     if (why.empty() && tile_masses == 0 && in.tile_cap == kWsDefaultTile && !pull_wanted(s)) {
         tg::WsLayout W{};
         ws_stage_layout(s->prec, tile_infos(s->plan), W);
@@ -723,7 +827,6 @@ std::string plan_scene(titan_gb300_sim *s, int tile_masses, tg::PlanInput &in) {
             why = tg::build_plan(in, s->plan);
         }
     }
-    s->plan_req = tile_masses;
     return why;
 }
 
@@ -955,6 +1058,25 @@ int build_device(titan_gb300_sim *s) {
         if (!(r.next = (int *)s->mem.get(sizeof(int), e))) return s->cuda_fail(e, "alloc bin queue");
     }
     DEVCOPY(a.halo, P.halo, "upload halo");
+    s->gargs = tg::GridResArgs{};
+    s->use_grid = !tiles_run.empty() && grid_wanted(s) && !s->use_pull &&
+                  choose_grid(s, tiles, s->grid_shape, s->gargs.stage, s->grid_smem);
+    if (s->use_grid) {
+        s->gargs.ntiles = (int32_t)tiles.size();
+        std::vector<int32_t> halo(P.halo);
+        std::vector<uint8_t> exported(np, 0);
+        for (int32_t &h : halo) {
+            if (!s->fixed.empty() && s->fixed[P.new2old[h]]) h = -1;
+            else exported[h] = 1;
+        }
+        if (s->use_rtiles) DEVCOPY(s->gargs.tiles, tiles, "upload tiles");
+        else s->gargs.tiles = a.tiles;
+        DEVCOPY(s->gargs.halo, halo, "upload halo");
+        DEVCOPY(s->gargs.exported, exported, "upload exported masses");
+        s->gargs.xbytes = np * tg::grid_resident_exchange_bytes(s->prec);
+        if (!(s->gargs.xbuf = (uint8_t *)s->mem.get(2 * s->gargs.xbytes, e))) return s->cuda_fail(e, "alloc exchange");
+        CK(cudaMemset(s->gargs.xbuf, 0, 2 * s->gargs.xbytes), "clear exchange");
+    }
     DEVCOPY(a.warp_inc_off, P.warp_inc_off, "upload warp offsets");
     std::vector<uint8_t> deg(np, 0);
     std::copy(P.deg.begin(), P.deg.end(), deg.begin());
@@ -1116,6 +1238,29 @@ cudaGraphExec_t get_graph(titan_gb300_sim *s, int len, int parity, cudaError_t &
 }
 
 bool ensure_device(titan_gb300_sim *s) { return cudaSetDevice(s->device) == cudaSuccess; }
+
+// Whether this call of step() is one resident-grid launch: two steps or more
+// (a launch stages the tiles' tables once).  Under stream capture the
+// per-step path decides, as without the resident grid.
+bool grid_runs(titan_gb300_sim *s, int64_t nsteps) {
+    if (!s->use_grid || nsteps < kGridMinSteps) return false;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+}
+
+// The host's clock and step count after nsteps steps.
+void advance_clock(titan_gb300_sim *s, int64_t nsteps) {
+    if (s->passes() == 2) {
+        const double h = 0.5 * s->dt;
+        for (int64_t i = 0; i < nsteps; i++) {  // src/sim.cu:1574-1583
+            s->T = s->T + h;
+            s->T = s->T + h;
+        }
+    } else {
+        for (int64_t i = 0; i < nsteps; i++) s->T = s->T + s->dt;  // src/sim.cu:1590
+    }
+    s->steps += nsteps;
+}
 
 // After a synchronisation: did a step kernel give up a bounded wait?
 int check_kernel_error(titan_gb300_sim *s) {
@@ -1645,6 +1790,21 @@ int titan_gb300_step(titan_gb300_sim *s, int64_t nsteps) try {
     if (nsteps == 0) return TITAN_GB300_OK;
     if (!ensure_device(s)) return s->fail(TITAN_GB300_ECUDA, "cudaSetDevice failed");
     cudaError_t e = cudaSuccess;
+    if (grid_runs(s, nsteps)) {
+        s->gargs.T0 = s->T;
+        const cudaError_t r = tg::launch_grid_resident(s->prec, s->integrator, s->args, s->gargs, s->grid_shape,
+                                                       s->grid_smem, s->parity, nsteps, 1, s->stream);
+        if (r == cudaSuccess) {
+            const int P = s->passes();
+            s->gargs.base += (uint32_t)(nsteps * P);
+            s->parity ^= (int)((nsteps * P) & 1);
+            advance_clock(s, nsteps);
+            return TITAN_GB300_OK;
+        }
+        if (r != cudaErrorCooperativeLaunchTooLarge) return s->cuda_fail(r, "launch resident grid");
+        cudaGetLastError();
+        s->use_grid = false;  // the device has less room than planned for: per-step kernels
+    }
     if (s->use_res)
         CK(tg::launch_resident(s->prec, s->args, s->rargs, s->res_ctas, s->res_threads, s->parity, nsteps, 1,
                                s->args.ntiles == 0, s->stream),
@@ -1696,16 +1856,7 @@ int titan_gb300_step(titan_gb300_sim *s, int64_t nsteps) try {
     // later work on the handle's stream sees the resident tiles' results
     if (!joined) CK(cudaStreamWaitEvent(s->stream, s->ev_join, 0), "join resident tiles");
     if (rc) return rc;
-    if (P == 2) {
-        const double h = 0.5 * s->dt;
-        for (int64_t i = 0; i < nsteps; i++) {  // src/sim.cu:1574-1583
-            s->T = s->T + h;
-            s->T = s->T + h;
-        }
-    } else {
-        for (int64_t i = 0; i < nsteps; i++) s->T = s->T + s->dt;  // src/sim.cu:1590
-    }
-    s->steps += nsteps;
+    advance_clock(s, nsteps);
     return TITAN_GB300_OK;
 } catch (...) {
     return host_exception(s);
@@ -1716,7 +1867,7 @@ int titan_gb300_prepare_steps(titan_gb300_sim *s, int64_t nsteps) try {
     if (s->serving) return s->fail(TITAN_GB300_ESTATE, "the scene is being stepped by a request server");
     if (!s->started) return s->fail(TITAN_GB300_ESTATE, "The simulation has not started.");
     if (nsteps < 0) return s->fail(TITAN_GB300_EINVAL, "negative step count");
-    if (s->args.ntiles == 0 || nsteps <= 1) return TITAN_GB300_OK;
+    if (s->args.ntiles == 0 || nsteps <= 1 || grid_runs(s, nsteps)) return TITAN_GB300_OK;
     if (!ensure_device(s)) return s->fail(TITAN_GB300_ECUDA, "cudaSetDevice failed");
     // the same chunk sequence step(nsteps) replays, from the current parity
     cudaError_t e = cudaSuccess;

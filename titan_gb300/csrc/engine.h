@@ -161,6 +161,20 @@ struct TileResArgs {
     int32_t stage;          // 1: slab, actuation and incidence records staged in shared memory once per launch
 };
 
+// Every tile of a scene on its own CTA for all steps of a call
+// (resident_grid.cu).
+struct GridResArgs {
+    const TileInfo *tiles;      // all tiles of the plan, in order
+    const int32_t *halo;        // StepArgs.halo with -1 for fixed masses
+    const uint8_t *exported;    // per mass: 1 when another tile's halo has it
+    uint8_t *xbuf;              // two exchange buffers of xbytes each, tags 0 at start
+    int64_t xbytes;
+    uint32_t base;              // passes done since start (tags are base + pass, counts wrap)
+    double T0;                  // T of the launch's first step
+    int32_t ntiles;
+    int32_t stage;              // 1: slab, actuation and incidence records in shared memory
+};
+
 // Per-mass gather / scatter between caller order and tiled order.
 struct XferArgs {
     const int32_t *old2new;
@@ -247,6 +261,17 @@ size_t tile_resident_smem_bytes(int precision, const TileInfo &ti, int stage);
 cudaError_t tile_resident_prepare(int precision, int mpt, int stage, size_t smem);
 int tile_resident_ctas_per_sm(int precision, int mpt, int stage, int threads, size_t smem);
 cudaError_t launch_tile_resident(int precision, const StepArgs &a, const TileResArgs &r, int mpt, int threads,
+                                 size_t smem, int parity, int64_t nsteps, int write_acc, cudaStream_t s);
+// All tiles at once (resident_grid.cu): shared memory of one tile; for each
+// launch shape its threads per CTA and the CTAs per SM its registers allow;
+// bytes of one mass in an exchange buffer; and the cooperative launch of
+// nsteps steps.
+constexpr int kGridShapes = 3;
+size_t grid_resident_smem_bytes(int precision, const TileInfo &ti, int stage);
+int grid_resident_threads(int shape);
+int grid_resident_ctas(int shape);
+int grid_resident_exchange_bytes(int precision);
+cudaError_t launch_grid_resident(int precision, int integ, const StepArgs &a, const GridResArgs &r, int shape,
                                  size_t smem, int parity, int64_t nsteps, int write_acc, cudaStream_t s);
 cudaError_t launch_gather(int precision, const XferArgs &a, cudaStream_t s);
 // float positions of all a.count masses in caller order into out (device)

@@ -25,13 +25,19 @@ __device__ __forceinline__ void comp_add_prod(float &hi, float &lo, float wh, fl
 }
 
 // INTEG: the integrator (INTEG_*) fixed at compile time, or -1 to read it
-// from prm at run time.
+// from prm at run time.  rk2_stage, rk0: RK2's half step and the step's
+// starting state, where the caller holds them (else a.rk2_stage, and the
+// record in out); acc0: VERLET's acceleration of the step before, kept by the
+// caller (else in a.acc, which is then written every step).
 template <int PREC, int INTEG = -1>
 __device__ __forceinline__ void integrate(const StepArgs &a, const TileInfo &ti, int64_t g, uint8_t fl,
                                           typename Real<PREC>::T m, typename Real<PREC>::T F0,
                                           typename Real<PREC>::T F1, typename Real<PREC>::T F2, St<PREC> &s,
                                           void *out, int64_t gs, int write_acc, int64_t np,
-                                          const DevParams *prm) {
+                                          const DevParams *prm, int rk2_stage = -1,
+                                          const St<PREC> *rk0 = nullptr,
+                                          typename Real<PREC>::T *acc0 = nullptr) {
+    const int half = rk2_stage >= 0 ? rk2_stage : a.rk2_stage;
     if constexpr (PREC == P_FP64) {
         double Fd[3] = {F0, F1, F2};
         const D3 gm = mul3_alu(prm->g, m);
@@ -69,14 +75,19 @@ __device__ __forceinline__ void integrate(const StepArgs &a, const TileInfo &ti,
         double *ac = reinterpret_cast<double *>(a.acc);
         const int integ = INTEG >= 0 ? INTEG : prm->integrator;
         if (integ == INTEG_VERLET) {  // src/sim.cu:1155-1159; acc is state
-            double ap[3] = {ac[g], ac[np + g], ac[2 * np + g]};
+            const double ap[3] = {acc0 ? acc0[0] : ac[g], acc0 ? acc0[1] : ac[np + g], acc0 ? acc0[2] : ac[2 * np + g]};
 #pragma unroll
             for (int c = 0; c < 3; c++) s.v[c] = s.v[c] + (0.5 * (ap[c] + acc[c])) * dt;
 #pragma unroll
             for (int c = 0; c < 3; c++) s.x[c] = s.x[c] + (s.v[c] * dt + (0.5 * acc[c]) * prm->dt2);
-            write_acc = 1;
+            if (acc0) {
+#pragma unroll
+                for (int c = 0; c < 3; c++) acc0[c] = acc[c];
+            } else {
+                write_acc = 1;
+            }
         } else if (integ == INTEG_RK2) {  // src/sim.cu:1141-1154
-            if (a.rk2_stage == 0) {
+            if (half == 0) {
 #pragma unroll
                 for (int c = 0; c < 3; c++) s.x[c] = s.x[c] + (0.5 * s.v[c]) * dt;
 #pragma unroll
@@ -84,7 +95,7 @@ __device__ __forceinline__ void integrate(const StepArgs &a, const TileInfo &ti,
             } else {
                 // the step's starting state is still this mass's record in
                 // the buffer this launch writes
-                const St<PREC> b = load_state<PREC>(out, gs);
+                const St<PREC> b = rk0 ? *rk0 : load_state<PREC>(out, gs);
 #pragma unroll
                 for (int c = 0; c < 3; c++) s.x[c] = b.x[c] + s.v[c] * dt;
 #pragma unroll
@@ -164,7 +175,7 @@ __device__ __forceinline__ void integrate(const StepArgs &a, const TileInfo &ti,
             // v += (a_prev + a) dt / 2;  x += v dt + a dt^2 / 2
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-                const float w = 0.5f * (ac[(int64_t)c * np + g] + acc[c]);
+                const float w = 0.5f * ((acc0 ? acc0[c] : ac[(int64_t)c * np + g]) + acc[c]);
                 const float r = (0.5f * acc[c]) * prm->dt2f;
                 if constexpr (PREC == P_FP32C) {
                     comp_add_prod(s.v[c], s.vl[c], w, 0.f, prm->dt_hi, prm->dt_lo, 0.f);
@@ -173,10 +184,11 @@ __device__ __forceinline__ void integrate(const StepArgs &a, const TileInfo &ti,
                     s.v[c] = s.v[c] + w * prm->dt_hi;
                     s.x[c] = s.x[c] + (s.v[c] * prm->dt_hi + r);
                 }
+                if (acc0) acc0[c] = acc[c];
             }
-            write_acc = 1;
+            if (!acc0) write_acc = 1;
         } else if (integ == INTEG_RK2) {
-            if (a.rk2_stage == 0) {
+            if (half == 0) {
                 // x += v dt / 2 (with the step's starting v);  v += a dt / 2
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
@@ -192,7 +204,7 @@ __device__ __forceinline__ void integrate(const StepArgs &a, const TileInfo &ti,
             } else {
                 // from the step's starting state, still this mass's record in
                 // the buffer this launch writes: x = x0 + v dt;  v = v0 + a dt
-                const St<PREC> b = load_state<PREC>(out, gs);
+                const St<PREC> b = rk0 ? *rk0 : load_state<PREC>(out, gs);
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
                     if constexpr (PREC == P_FP32C) {

@@ -603,7 +603,7 @@ static std::string build_plan_tables(const PlanInput &in, Plan &P) {
     P.ns = ns;
     if (n <= 0) return "no masses";
     if (n >= (int64_t(1) << 31) - 1) return "more than 2^31-2 masses";
-    if (in.tile_cap < 32 || in.tile_cap > 2048) return "tile size must be in [32, 2048]";
+    if (in.tile_cap < in.tile_min || in.tile_cap > 2048) return "tile size must be in [32, 2048]";
     if (in.heavy_threshold < 1 || in.heavy_threshold > 254) return "heavy threshold must be in [1, 254]";
 
     // ---- bodies --------------------------------------------------------
