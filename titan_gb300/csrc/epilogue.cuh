@@ -61,13 +61,10 @@ __device__ __forceinline__ void integrate(const StepArgs &a, const TileInfo &ti,
         }
         if (fl & MF_LOCAL) local_apply(a, g, s.x, s.v, Fd);
         if (fl & MF_DRAG) {  // src/sim.cu:1134-1137
-            double vn = nrm3(s.v[0], s.v[1], s.v[2]);
-            if (vn != 0.0) {
-                double c = (double)(-a.drag[g]) * (vn * vn);
-                Fd[0] = Fd[0] + (s.v[0] * c) / vn;
-                Fd[1] = Fd[1] + (s.v[1] * c) / vn;
-                Fd[2] = Fd[2] + (s.v[2] * c) / vn;
-            }
+            const D3 q = drag_added(s.v[0], s.v[1], s.v[2], a.drag[g], Fd[0], Fd[1], Fd[2]);
+            Fd[0] = q.x;
+            Fd[1] = q.y;
+            Fd[2] = q.z;
         }
         const double dt = prm->dt;
         const D3 fm = div3_alu(Fd, m);
@@ -151,11 +148,10 @@ __device__ __forceinline__ void integrate(const StepArgs &a, const TileInfo &ti,
             }
             if (fl & MF_LOCAL) local_apply(a, g, x, v, Fd);
             if (fl & MF_DRAG) {
-                double vn = nrm3(v[0], v[1], v[2]);
-                if (vn != 0.0) {
-                    double c = (double)(-a.drag[g]) * (vn * vn);
-                    for (int k = 0; k < 3; k++) Fd[k] = Fd[k] + (v[k] * c) / vn;
-                }
+                const D3 q = drag_added(v[0], v[1], v[2], a.drag[g], Fd[0], Fd[1], Fd[2]);
+                Fd[0] = q.x;
+                Fd[1] = q.y;
+                Fd[2] = q.z;
             }
             for (int c = 0; c < 3; c++) {
                 Ff[c] = (float)Fd[c];

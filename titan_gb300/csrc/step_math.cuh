@@ -67,35 +67,59 @@ __device__ __forceinline__ D3 div3_alu(const double *a, double b) {
     return alu_bad(bad) || !alu_nonzero(y) ? div3_wide(a[0], a[1], a[2], b) : r;
 }
 
-// src/object.cu:73-106
-__device__ __forceinline__ void plane_apply(const double *n, double off, double fk, double fs,
-                                            const double *x, const double *v, double *F) {
-    double disp = dot3_alu(x, n) - off;
-    if (!(disp < 0)) return;  // only zeros would be added otherwise
-    double fdn = dot3(F, n);
-    double fn[3] = {n[0] * fdn, n[1] * fdn, n[2] * fdn};
+// The force on a mass below a plane, from the force F so far.  Out of line:
+// most warps have no mass in contact.  On the FP64 pipe its square roots and
+// divisions were 5 us of a step of the 5^3 robot standing on its plane (10.0
+// -> 6.5 us).
+__device__ __noinline__ D3 plane_contact(double n0, double n1, double n2, double disp, double fk, double fs, double v0,
+                                         double v1, double v2, double F0, double F1, double F2) {
+    const double n[3] = {n0, n1, n2}, v[3] = {v0, v1, v2};
+    double F[3] = {F0, F1, F2};
+    const D3 fn3 = mul3_alu(n, dot3_alu(F, n));
     if (fs > 0 || fk > 0) {
-        double vdn = dot3(v, n);
-        double vp[3] = {v[0] - n[0] * vdn, v[1] - n[1] * vdn, v[2] - n[2] * vdn};
-        double vn = nrm3(vp[0], vp[1], vp[2]);
+        const D3 nv = mul3_alu(n, dot3_alu(v, n));
+        const double vp[3] = {v[0] - nv.x, v[1] - nv.y, v[2] - nv.z};
+        const double vn = nrm3_alu(vp[0], vp[1], vp[2]);
         if (vn > 1e-16) {
-            double fmag = fk * nrm3(fn[0], fn[1], fn[2]);
-            F[0] = F[0] - (vp[0] * fmag) / vn;
-            F[1] = F[1] - (vp[1] * fmag) / vn;
-            F[2] = F[2] - (vp[2] * fmag) / vn;
+            const D3 t = mul3_alu(vp, fk * nrm3_alu(fn3.x, fn3.y, fn3.z));
+            const double tv[3] = {t.x, t.y, t.z};
+            const D3 q = div3_alu(tv, vn);
+            F[0] = F[0] - q.x;
+            F[1] = F[1] - q.y;
+            F[2] = F[2] - q.z;
         } else {
-            double fp[3] = {F[0] - fn[0], F[1] - fn[1], F[2] - fn[2]};
-            if (fs * nrm3(fn[0], fn[1], fn[2]) > nrm3(fp[0], fp[1], fp[2])) {
+            const double fp[3] = {F[0] - fn3.x, F[1] - fn3.y, F[2] - fn3.z};
+            if (fs * nrm3_alu(fn3.x, fn3.y, fn3.z) > nrm3_alu(fp[0], fp[1], fp[2])) {
                 F[0] = F[0] - fp[0];
                 F[1] = F[1] - fp[1];
                 F[2] = F[2] - fp[2];
             }
         }
     }
-    double s = (-disp) * kNormal;
-    F[0] = F[0] + n[0] * s;
-    F[1] = F[1] + n[1] * s;
-    F[2] = F[2] + n[2] * s;
+    const D3 q = mul3_alu(n, (-disp) * kNormal);
+    return D3{F[0] + q.x, F[1] + q.y, F[2] + q.z};
+}
+
+// src/object.cu:73-106
+__device__ __forceinline__ void plane_apply(const double *n, double off, double fk, double fs,
+                                            const double *x, const double *v, double *F) {
+    double disp = dot3_alu(x, n) - off;
+    if (!(disp < 0)) return;  // only zeros would be added otherwise
+    const D3 r = plane_contact(n[0], n[1], n[2], disp, fk, fs, v[0], v[1], v[2], F[0], F[1], F[2]);
+    F[0] = r.x;
+    F[1] = r.y;
+    F[2] = r.z;
+}
+
+// F with the drag of a mass at velocity v added (src/sim.cu:1134-1137).
+__device__ __noinline__ D3 drag_added(double v0, double v1, double v2, int32_t drag, double F0, double F1, double F2) {
+    const double v[3] = {v0, v1, v2};
+    const double vn = nrm3_alu(v0, v1, v2);
+    if (!(vn != 0.0)) return D3{F0, F1, F2};
+    const D3 t = mul3_alu(v, (double)(-drag) * (vn * vn));
+    const double tv[3] = {t.x, t.y, t.z};
+    const D3 q = div3_alu(tv, vn);
+    return D3{F0 + q.x, F1 + q.y, F2 + q.z};
 }
 
 // src/object.cu:53-56
