@@ -586,13 +586,12 @@ tg::PlanInput plan_input(titan_gb300_sim *s, int tile_masses, bool grid = false)
     in.type = s->type.empty() ? nullptr : s->type.data();
     in.nbodies = s->body_ptr.empty() ? 0 : (int64_t)s->body_ptr.size() - 1;
     in.body_ptr = s->body_ptr.empty() ? nullptr : s->body_ptr.data();
-    // Default tile.  Large scenes: 256 masses in FP64 (with two threads per
-    // mass: the FP64 pipe wants the warps; 2.40 ms per 100^3 step against
-    // 2.50 with tiles of 128), 208 for the FP32 forms' warp-specialised
+    // Default tile.  Large scenes: 96 masses in FP64 (three CTAs per SM,
+    // step_var.cu; 256 where a form was chosen), 208 for the FP32 forms' warp-specialised
     // kernel (two stages fit one SM's shared memory; 192 where they would
     // not, plan_scene) and 256 for the per-tile forms.  Smaller scenes get
     // smaller tiles so that their tiles cover the SMs: FP64 about 1.6 tiles
-    // per SM (tiles of 32 to 256 masses), the warp-specialised form about
+    // per SM (tiles of 32 to 96 masses), the warp-specialised form about
     // 4 (64 to 208).  In the FP32 forms a body that fits the large-scene
     // tile stays whole (a halo-free tile runs resident: 2.0 us per step for
     // the 5^3 lattice against 3.3 split in four); in FP64, bound by each
@@ -611,7 +610,7 @@ tg::PlanInput plan_input(titan_gb300_sim *s, int tile_masses, bool grid = false)
             return (int)std::max<int64_t>(lo, std::min<int64_t>(hi, t));
         };
         if (s->prec == P_FP64) {
-            in.tile_cap = fit(1.6, 32, 256);  // small bodies split too: FP64 binds per SM
+            in.tile_cap = fit(1.6, 32, grid_wanted(s) ? 96 : 256);  // small bodies split too: FP64 binds per SM
         } else if (pull) {
             in.tile_cap = fit(4.0, 64, kPullDefaultTile);
             in.whole_cap = kPullDefaultTile;
@@ -857,6 +856,9 @@ int build_device(titan_gb300_sim *s) {
     s->threads = s->threads_req > 0 ? s->threads_req
                                     : std::max(min_threads, std::min(512, ((P.max_nm + 31) / 32) * 32 *
                                                                               (s->prec == P_FP64 ? 2 : 1)));
+    // 96-mass FP64 tiles, three CTAs per SM: 196 us per 60^3 step with 256
+    // threads, 214 with 192
+    if (s->prec == P_FP64 && s->threads_req == 0 && P.max_nm > 64) s->threads = std::max(s->threads, 256);
     s->npad = ((s->n + 127) / 128) * 128;
     const int64_t np = s->npad;
     auto &a = s->args;
@@ -1022,6 +1024,7 @@ int build_device(titan_gb300_sim *s) {
                 return s->fail(TITAN_GB300_EINVAL, "3 or 4 CTAs per SM need at most 256 threads per CTA");
             s->step_variant = s->min_ctas_req == 3 ? 1 : 2;
         }
+        if (s->prec == P_FP64 && s->threads <= 256 && (int64_t)tiles_run.size() > 2 * sms_dev) s->step_variant = 3;
         if (s->use_async)
             CK(tg::step_async_prepare(s->prec, s->smem), "set shared memory");
         else

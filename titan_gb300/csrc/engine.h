@@ -214,10 +214,9 @@ int state_words(int precision);
 // dynamic shared memory of one tile's CTA
 size_t tile_smem_bytes(int precision, int slots, int entries, int heavy);
 // Per-tile kernel, launch-bound variant 0: (512 threads, 1 CTA/SM), every
-// precision; FP32 forms also 1: (256, 3) and 2: (256, 4) -- at most 256
-// threads per CTA, registers capped for 3 or 4 resident CTAs per SM.
-constexpr int kStepVariants = 3;
-const void *step_kernel_capped(int precision, int variant);  // null if not compiled
+// precision; FP32 forms also 1: (256, 3) and 2: (256, 4), FP64 3: (256, 3) --
+// at most 256 threads per CTA, registers capped for 3 or 4 resident CTAs per SM.
+const void *step_kernel_capped(int precision, int variant, int integ);  // null if not compiled
 cudaError_t step_prepare(int precision, int variant, int integ, size_t smem);
 cudaError_t launch_step(int precision, int variant, int integ, const StepArgs &a, int ntiles, int threads,
                         size_t smem, int parity, int write_acc, cudaStream_t s);

@@ -123,7 +123,6 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
     constexpr int kBatch = PREC == P_FP64 ? 1 : 4;
     constexpr int kChunks = PREC == P_FP32 ? 2 : 4;  // of one record in the exchange
     constexpr int kPoll = 4;                         // chunks a thread has in flight
-    constexpr int kWords = PREC == P_FP64 ? 7 : 0;  // incidence words kept in registers (FP32: they would spill)
     extern __shared__ __align__(16) uint8_t smem[];
     const DevParams *prm = reinterpret_cast<const DevParams *>(smem);
     for (int v = threadIdx.x; v < (int)(kParamBytes / 16); v += blockDim.x)
@@ -172,7 +171,6 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
         m = __ldg(reinterpret_cast<const R *>(a.mass) + g_own);
         woff = __ldg(a.warp_inc_off + ti.warp_off + (i_own >> 5)) - inc_base;
     }
-    uint2 cw[kWords > 0 ? kWords : 1];
     // FP64: the sum of component c of mass ic, in the warp that has it, where
     // there is a thread for each (step_kernel.cuh)
     const int nmp = (nm + 31) & ~31;
@@ -186,16 +184,11 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
         woff_sp = __ldg(a.warp_inc_off + ti.warp_off + (i_sp >> 5)) - inc_base;
     }
 
-    // the thread's incidence words, constant over the steps
-    const uint32_t d_c = split ? d_sp : (d == 255 ? 0 : d);
-    const uint2 *const ip = reinterpret_cast<const uint2 *>(a.inc + (split ? woff_sp : woff) + inc_base) +
+    // the thread's incidence words
+    const uint32_t d_c = split ? d_sp : (d == 255 ? 0 : d), nw = (d_c + 3) >> 2, pad = (uint32_t)E * 0x10001u;
+    const uint2 *const ip = reinterpret_cast<const uint2 *>(incb + (split ? woff_sp : woff)) +
                             ((split ? i_sp : i_own) & 31);
-    const uint32_t nw = (d_c + 3) >> 2;
-#pragma unroll
-    for (int w = 0; w < kWords; w++)
-        if ((uint32_t)w < nw) cw[w] = __ldg(ip + 32 * w);
-    const uint2 *const ips = reinterpret_cast<const uint2 *>(incb + (split ? woff_sp : woff)) +
-                             ((split ? i_sp : i_own) & 31);
+    auto word = [&](uint32_t w) { return w >= nw ? make_uint2(pad, pad) : STAGE ? ip[32 * w] : __ldg(ip + 32 * w); };
 
     // the host's clock: the time record may already be the launch's last
     // (written by CTA 0) when a CTA far from it starts
@@ -290,12 +283,7 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
         }
             if (split) {
             if (i_sp < nm) {
-                double F = 0;
-#pragma unroll
-                for (int w = 0; w < kWords; w++)
-                    if ((uint32_t)w < nw) F = gather_word_component(slots, cw[w], c_sp, F);
-                for (uint32_t w = kWords; w < nw; w++)
-                    F = gather_word_component(slots, STAGE ? ips[32 * w] : __ldg(ips + 32 * w), c_sp, F);
+                const double F = gather_list_component(slots, nw, word, c_sp);
                 sF[c_sp * nm + i_sp] = F;
             }
             __syncthreads();
@@ -313,11 +301,7 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
                 F1 = (R)sF[nm + i_own];
                 F2 = (R)sF[2 * nm + i_own];
             } else {
-#pragma unroll
-                for (int w = 0; w < kWords; w++)
-                    if ((uint32_t)w < nw) gather_word_padded<PREC>(slots, cw[w], F0, F1, F2);
-                for (uint32_t w = kWords; w < nw; w++)
-                    gather_word_padded<PREC>(slots, STAGE ? ips[32 * w] : __ldg(ips + 32 * w), F0, F1, F2);
+                for (uint32_t w = 0; w < nw; w++) gather_word_padded<PREC>(slots, word(w), F0, F1, F2);
             }
             St<PREC> s = load_state_smem<PREC>(st, i_own);
             const int rk2_stage = INTEG == INTEG_RK2 ? (int)(pass & 1) : 0;

@@ -44,10 +44,11 @@ const void *step_kernel_default(int integ) {
     }
 }
 
-// The register-capped variants exist for Euler in the FP32 forms; other
-// requests run the default launch bounds.
+// The register-capped variants exist for Euler in the FP32 forms (1, 2) and
+// for FP64 (3); other requests run the default launch bounds.
 const void *step_kernel(int precision, int variant, int integ) {
-    if (variant != 0 && precision != P_FP64 && integ == INTEG_EULER) return step_kernel_capped(precision, variant);
+    if (precision == P_FP64 ? variant == 3 : variant != 0 && integ == INTEG_EULER)
+        return step_kernel_capped(precision, variant, integ);
     return precision == P_FP64   ? step_kernel_default<P_FP64>(integ)
            : precision == P_FP32 ? step_kernel_default<P_FP32>(integ)
                                  : step_kernel_default<P_FP32C>(integ);

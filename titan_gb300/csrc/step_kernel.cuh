@@ -43,7 +43,7 @@ __host__ __device__ constexpr int prefetch_w() { return LBM >= 3 ? 0 : 7; }
 
 // slab entries in flight per thread in phase B (FP64 records are 32 B)
 template <int PREC, int LBM>
-__host__ __device__ constexpr int batch_b() { return (PREC == P_FP64 || LBM >= 3) ? 2 : 4; }
+__host__ __device__ constexpr int batch_b() { return PREC == P_FP64 ? (LBM >= 3 ? 1 : 2) : (LBM >= 3) ? 2 : 4; }
 
 template <int PREC>
 __host__ __device__ constexpr int rec_bytes() { return PREC == P_FP32 ? 32 : 48; }
@@ -184,16 +184,9 @@ __device__ __forceinline__ void tile_step(const StepArgs &a, const TileInfo &ti,
             if (d != 255) {
                 const uint2 *ip =
                     reinterpret_cast<const uint2 *>(a.inc + __ldg(a.warp_inc_off + ti.warp_off + (i >> 5))) + (i & 31);
-                const uint32_t nw = (d + 3) >> 2;
-                for (uint32_t w0 = 0; w0 < nw; w0 += kBatchC) {
-                    uint2 cw[kBatchC];
-#pragma unroll
-                    for (int k = 0; k < kBatchC; k++)
-                        if (w0 + k < nw) cw[k] = __ldg(ip + 32 * (w0 + k));
-#pragma unroll
-                    for (int k = 0; k < kBatchC; k++)
-                        if (w0 + k < nw) F = gather_word_component(slots, cw[k], c, F);
-                }
+                const uint32_t nw = (d + 3) >> 2, pad = (uint32_t)E * 0x10001u;
+                F = gather_list_component(
+                    slots, nw, [&](uint32_t w) { return w < nw ? __ldg(ip + 32 * w) : make_uint2(pad, pad); }, c);
             }
             sF[c * ti.nm + i] = F;
         }

@@ -68,9 +68,7 @@ __device__ __forceinline__ D3 div3_alu(const double *a, double b) {
 }
 
 // The force on a mass below a plane, from the force F so far.  Out of line:
-// most warps have no mass in contact.  On the FP64 pipe its square roots and
-// divisions were 5 us of a step of the 5^3 robot standing on its plane (10.0
-// -> 6.5 us).
+// most warps have no mass in contact.
 __device__ __noinline__ D3 plane_contact(double n0, double n1, double n2, double disp, double fk, double fs, double v0,
                                          double v1, double v2, double F0, double F1, double F2) {
     const double n[3] = {n0, n1, n2}, v[3] = {v0, v1, v2};

@@ -142,8 +142,11 @@ __device__ __forceinline__ double actuated_rest_f64(double rest, double amp, dou
 }
 
 // FP64 force: the reference's operations in the reference's order, the
-// additions on the FP64 pipe, the square root, divisions and products on the
-// integer units (fp64_alu.cuh: the same bits).
+// additions and the product with k on the FP64 pipe, the square root, the
+// divisions and the other products on the integer units (fp64_alu.cuh: the
+// same bits).  Both are then about equally busy: the products w_i u_i or
+// u_i dd moved to the FP64 pipe cost 2 and 4 % of a 60^3 step, the sums of
+// |d|^2 or of w.u moved off it 3 and 7 %.
 __device__ __forceinline__ F3<P_FP64> spring_force_f64(int sa, int sb, double k, double rs, double damping,
                                                        const uint8_t *st) {
     const double2 *pa = reinterpret_cast<const double2 *>(st + (int64_t)sa * 48);
@@ -155,8 +158,7 @@ __device__ __forceinline__ F3<P_FP64> spring_force_f64(int sa, int sb, double k,
     const Alu n2 = alu_unpack((alu_pack(alu_square(d0)) + alu_pack(alu_square(d1))) + alu_pack(alu_square(d2)), bad);
     AluDivisor nd;
     const double nrm = alu_pack(alu_sqrt(n2, nd));
-    Alu fs = alu_mul(alu_unpack(k, bad), alu_unpack(rs - nrm, bad));
-    alu_carry(fs);
+    const Alu fs = alu_unpack(k * (rs - nrm), bad);
     const Alu u0 = alu_div(d0, nd), u1 = alu_div(d1, nd), u2 = alu_div(d2, nd);
     double f0 = alu_pack(alu_mul(u0, fs)), f1 = alu_pack(alu_mul(u1, fs)), f2 = alu_pack(alu_mul(u2, fs));
     if (damping != 0.0) {
@@ -301,15 +303,31 @@ __device__ __forceinline__ void gather_word_padded(const uint8_t *slots, uint2 c
     }
 }
 
-// One component (0, 1, 2) of the FP64 forces that a whole word's codes name,
-// added in the same order.
-__device__ __forceinline__ double gather_word_component(const uint8_t *slots, uint2 cw, int c, double F) {
-#pragma unroll
-    for (int h = 0; h < 4; h++) {
-        const uint32_t word = h < 2 ? cw.x : cw.y;
-        const uint32_t code = (h & 1) ? (word >> 16) : (word & 0xffffu);
-        const double f = *reinterpret_cast<const double *>(slots + (int64_t)(code & 0x7fff) * 32 + 8 * c);
-        F = F + __hiloint2double(__double2hiint(f) ^ (int)((code & 0x8000u) << 16), __double2loint(f));
+// FP64: component comp of the sum over a whole incidence list of nw words, in
+// the same order, the slots of the next word loaded while this one's are added
+// (9^3 lattice: 7.35 -> 7.1 us per step; in the FP32 forms, whose additions are
+// short, it changed nothing).  word(w): the list's word w, and for w past its
+// end the code of the zero slot.
+template <class Word>
+__device__ __forceinline__ double gather_list_component(const uint8_t *slots, uint32_t nw, Word word, int comp) {
+    auto slot = [&](uint32_t code) {
+        return *reinterpret_cast<const double *>(slots + (int64_t)(code & 0x7fffu) * 32 + 8 * comp);
+    };
+    uint2 c = word(0), n = word(1);
+    double f0 = slot(c.x), f1 = slot(c.x >> 16), f2 = slot(c.y), f3 = slot(c.y >> 16), F = 0;
+    for (uint32_t w = 0; w < nw; w++) {
+        const uint2 n2 = word(w + 2);
+        const double g0 = slot(n.x), g1 = slot(n.x >> 16), g2 = slot(n.y), g3 = slot(n.y >> 16);
+        auto add = [&](uint32_t code, double f) {
+            F = F + __hiloint2double(__double2hiint(f) ^ (int)((code & 0x8000u) << 16), __double2loint(f));
+        };
+        add(c.x, f0);
+        add(c.x >> 16, f1);
+        add(c.y, f2);
+        add(c.y >> 16, f3);
+        f0 = g0, f1 = g1, f2 = g2, f3 = g3;
+        c = n;
+        n = n2;
     }
     return F;
 }
