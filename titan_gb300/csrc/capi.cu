@@ -114,11 +114,19 @@ struct titan_gb300_sim {
     int32_t *d_old2new = nullptr;
     double *d_xfer = nullptr;     // 9n doubles
     int64_t *d_idx = nullptr;     // n
-    double *h_xfer = nullptr;     // pinned 9n doubles
+    double *h_xfer = nullptr;     // pinned 9n doubles, then the error flag k_gather copies
+    int *h_err = nullptr;
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
     // diagnostics (lazy)
     int32_t *d_sl = nullptr, *d_sr = nullptr;
-    double *d_sk = nullptr, *d_srest = nullptr, *d_partials = nullptr, *d_dout = nullptr;
+    double *d_partials = nullptr, *d_dout = nullptr;
+    // spring parameters on the device in creation order (k, rest, damping,
+    // omega, amp, phase), each there once something needs it; sp_current: it
+    // holds the host array's values.  d_espring: the spring of each slab entry.
+    enum { SP_K, SP_REST, SP_DAMPING, SP_OMEGA, SP_AMP, SP_PHASE, SP_COUNT };
+    double *d_sp[SP_COUNT] = {};
+    bool sp_current[SP_COUNT] = {};
+    int32_t *d_espring = nullptr;
 
     size_t rsize() const { return prec == P_FP64 ? sizeof(double) : sizeof(float); }
     int comps() const { return tg::state_words(prec); }
@@ -191,8 +199,11 @@ struct titan_gb300_sim {
         mem.release();
         if (h_xfer) cudaFreeHost(h_xfer);
         h_xfer = nullptr;
+        h_err = nullptr;
         d_sl = d_sr = nullptr;
-        d_sk = d_srest = d_partials = d_dout = nullptr;
+        d_partials = d_dout = nullptr;
+        for (int q = 0; q < SP_COUNT; q++) d_sp[q] = nullptr, sp_current[q] = false;
+        d_espring = nullptr;
     }
     ~titan_gb300_sim() {
         if (stream) cudaStreamSynchronize(stream);
@@ -215,6 +226,17 @@ namespace {
         if (e_ != cudaSuccess) return s->cuda_fail(e_, what); \
     } while (0)
 
+// A page-locked host buffer's address on the device (cudaMallocHost or
+// cudaHostRegister), null for other memory.
+void *host_on_device(const void *p) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+}
+
 // Whether a caller's host buffer is page-locked (cudaMallocHost or
 // cudaHostRegister): such buffers are copied by DMA directly, without the
 // staging copy through the handle's own pinned buffer.
@@ -230,9 +252,10 @@ bool host_pinned(const void *p) {
 
 // memcpy of large host buffers split over a few threads (the staging copies
 // of whole-scene state are tens of MB; one core copies them at a fraction of
-// the host memory bandwidth).
+// the host memory bandwidth, and a new destination's pages are first touched
+// here: 15 MB of velocities into a new array took 1.39 ms with pieces of 8 MB).
 void par_memcpy(void *dst, const void *src, size_t bytes) {
-    constexpr size_t kPiece = 8u << 20;
+    constexpr size_t kPiece = 2u << 20;
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     const size_t nt = std::min<size_t>(std::min<size_t>(8, hw), (bytes + kPiece - 1) / kPiece);
     if (nt <= 1) {
@@ -829,6 +852,43 @@ std::string plan_scene(titan_gb300_sim *s, int tile_masses, tg::PlanInput &in) {
     return why;
 }
 
+// The device's copy of spring parameter q brought up to date with host.
+int upload_spring_array(titan_gb300_sim *s, int q, const std::vector<double> &host) {
+    cudaError_t e = cudaSuccess;
+    if (!s->d_sp[q] && !(s->d_sp[q] = (double *)s->mem.get(std::max<size_t>(1, host.size()) * 8, e)))
+        return s->cuda_fail(e, "alloc spring parameters");
+    if (!s->sp_current[q] && !host.empty())
+        CK(cudaMemcpyAsync(s->d_sp[q], host.data(), host.size() * 8, cudaMemcpyHostToDevice, s->stream),
+           "upload spring parameters");
+    s->sp_current[q] = true;
+    return TITAN_GB300_OK;
+}
+
+// The slab's records rewritten on the device for the parameters given (a bit
+// per SP_*), every spring's.  The host loop that builds all records and the
+// two copies it needs took 1.5 ms for the 137,000 springs of a 23^3 design.
+int refresh_entries(titan_gb300_sim *s, unsigned given) {
+    const tg::Plan &P = s->plan;
+    cudaError_t e = cudaSuccess;
+    if (!s->d_espring) {
+        std::vector<int32_t> es(P.ent_spring.begin(), P.ent_spring.end());
+        if (!(s->d_espring = dev_copy(s, es, e))) return s->cuda_fail(e, "upload entry springs");
+    }
+    const std::vector<double> *host[] = {&s->k, &s->rest, &s->damping, &s->omega, &s->amp, &s->phase};
+    tg::EntryArgs x{};
+    x.spring = s->d_espring;
+    x.rec = const_cast<void *>(s->args.ent);
+    x.act = const_cast<void *>(s->args.act);
+    x.count = (int64_t)P.ent_spring.size();
+    for (int q = 0; q < titan_gb300_sim::SP_COUNT; q++) {
+        if (!(given >> q & 1)) continue;
+        if (int rc = upload_spring_array(s, q, *host[q])) return rc;
+        x.par[q] = s->d_sp[q];
+    }
+    CK(tg::launch_entries(s->prec, x, s->stream), "refresh entries");
+    return TITAN_GB300_OK;
+}
+
 // Builds the plan and all device buffers; positions/velocities come from the
 // host mirror.  Keeps T / steps.
 int build_device(titan_gb300_sim *s) {
@@ -1122,7 +1182,8 @@ int build_device(titan_gb300_sim *s) {
     a.err = s->d_err;
     if (!(s->d_xfer = (double *)s->mem.get(9 * (size_t)s->n * 8, e))) return s->cuda_fail(e, "alloc staging");
     if (!(s->d_idx = (int64_t *)s->mem.get((size_t)s->n * 8, e))) return s->cuda_fail(e, "alloc staging");
-    CK(cudaMallocHost(&s->h_xfer, 9 * (size_t)s->n * 8), "alloc pinned staging");
+    CK(cudaMallocHost(&s->h_xfer, 9 * (size_t)s->n * 8 + 16), "alloc pinned staging");
+    s->h_err = reinterpret_cast<int *>(s->h_xfer + 9 * s->n);
     CK(cudaMemset(a.state0, 0, s->comps() * np * rs), "clear state");
     CK(cudaMemset(a.state1, 0, s->comps() * np * rs), "clear state");
     CK(cudaMemset(a.acc, 0, 3 * np * rs), "clear acc");
@@ -2026,25 +2087,32 @@ int titan_gb300_get_masses(titan_gb300_sim *s, int64_t count, const int64_t *idx
         CK(cudaMemcpyAsync(s->d_idx, idx, count * 8, cudaMemcpyHostToDevice, s->stream), "upload index");
         x.idx = s->d_idx;
     }
-    x.pos = pos ? s->d_xfer : nullptr;
-    x.vel = vel ? s->d_xfer + 3 * count : nullptr;
-    x.accout = acc ? s->d_xfer + 6 * count : nullptr;
-    // only the requested arrays come back: into a pinned caller buffer by
-    // DMA directly, else through the handle's pinned staging buffer
-    double *outs[3] = {pos, vel, acc};
+    // only the requested arrays come back: the kernel writes them into a
+    // page-locked caller buffer, else into the handle's staging buffer, and
+    // the error flag beside that
+    double *outs[3] = {pos, vel, acc}, *dst[3] = {nullptr, nullptr, nullptr};
     bool direct[3] = {false, false, false};
-    if (pos || vel || acc) {
-        CK(tg::launch_gather(s->prec, x, s->stream), "gather");
+    double *const stage = (double *)host_on_device(s->h_xfer);
+    int *const err_dst = (int *)host_on_device(s->h_err);
+    const bool any = pos || vel || acc;
+    if (any) {
+        if (!stage || !err_dst) return s->fail(TITAN_GB300_ECUDA, "the staging buffer is not mapped");
         for (int q = 0; q < 3; q++) {
             if (!outs[q]) continue;
-            direct[q] = host_pinned(outs[q]);
-            double *dst = direct[q] ? outs[q] : s->h_xfer + 3 * q * count;
-            CK(cudaMemcpyAsync(dst, s->d_xfer + 3 * q * count, 3 * count * 8, cudaMemcpyDeviceToHost, s->stream),
-               "download");
+            double *const h = (double *)host_on_device(outs[q]);
+            direct[q] = h && (reinterpret_cast<uintptr_t>(h) & 7) == 0;
+            dst[q] = direct[q] ? h : stage + 3 * q * count;
         }
+        x.pos = dst[0];
+        x.vel = dst[1];
+        x.accout = dst[2];
+        x.err = s->d_err;
+        x.err_out = err_dst;
+        CK(tg::launch_gather(s->prec, x, s->stream), "gather");
     }
     CK(cudaStreamSynchronize(s->stream), "download");
-    if (int rc = check_kernel_error(s)) return rc;
+    if (!any || *s->h_err)
+        if (int rc = check_kernel_error(s)) return rc;
     for (int q = 0; q < 3; q++)
         if (outs[q] && !direct[q]) par_memcpy(outs[q], s->h_xfer + 3 * q * count, 3 * count * 8);
     if (T) mass_times(s, idx, count, T);
@@ -2176,39 +2244,45 @@ int titan_gb300_set_spring_params(titan_gb300_sim *s, int64_t count, const int64
         if (j < 0 || j >= s->ns) return s->fail(TITAN_GB300_EINVAL, "spring index out of range");
         if (type && (type[q] < 0 || type[q] > 3)) return s->fail(TITAN_GB300_EINVAL, "spring type must be 0..3");
     }
-    for (int64_t q = 0; q < count; q++) {
-        int64_t j = idx ? idx[q] : q;
-        if (k) s->k[j] = k[q];
-        if (rest) s->rest[j] = rest[q];
-        if (damping) s->damping[j] = damping[q];
-        if (type) {
-            if (s->type.empty()) s->type.assign(s->ns, 0);
+    if (s->started) {  // what the stream still has to do reads the host arrays
+        if (!ensure_device(s)) return s->fail(TITAN_GB300_ECUDA, "cudaSetDevice failed");
+        CK(cudaStreamSynchronize(s->stream), "set springs");
+    }
+    if (omega && s->omega.empty()) s->omega.assign(s->ns, 0.0);
+    if (amp && s->amp.empty()) s->amp.assign(s->ns, 0.2);
+    if (phase && s->phase.empty()) s->phase.assign(s->ns, 0.0);
+    const double *in[] = {k, rest, damping, omega, amp, phase};
+    std::vector<double> *host[] = {&s->k, &s->rest, &s->damping, &s->omega, &s->amp, &s->phase};
+    unsigned given = 0;
+    for (int q = 0; q < titan_gb300_sim::SP_COUNT; q++) {
+        if (!in[q] || count == 0) continue;
+        given |= 1u << q;
+        s->sp_current[q] = false;
+        if (idx)
+            for (int64_t i = 0; i < count; i++) (*host[q])[idx[i]] = in[q][i];
+        else
+            par_memcpy(host[q]->data(), in[q], count * 8);
+    }
+    bool retyped = false;
+    if (type) {
+        if (s->type.empty()) s->type.assign(s->ns, 0);
+        for (int64_t q = 0; q < count; q++) {
+            int64_t j = idx ? idx[q] : q;
             bool was = s->type[j] >= 2, now = type[q] >= 2;
             if (was != now) replan = true;
+            retyped |= s->type[j] != type[q];
             s->type[j] = type[q];
-        }
-        if (omega) {
-            if (s->omega.empty()) s->omega.assign(s->ns, 0.0);
-            s->omega[j] = omega[q];
-        }
-        if (amp) {
-            if (s->amp.empty()) s->amp.assign(s->ns, 0.2);
-            s->amp[j] = amp[q];
-        }
-        if (phase) {
-            if (s->phase.empty()) s->phase.assign(s->ns, 0.0);
-            s->phase[j] = phase[q];
         }
     }
     if (!s->started) return TITAN_GB300_OK;
-    if (!ensure_device(s)) return s->fail(TITAN_GB300_ECUDA, "cudaSetDevice failed");
-    CK(cudaStreamSynchronize(s->stream), "set springs");
     if (replan) {
         int rc = pull_state(s);
         if (rc) return rc;
         s->drop_graphs();
         return build_device(s);
     }
+    // whole arrays and no new types: the device rewrites the slab records
+    if (!idx && !retyped && !s->use_res && !s->use_pull) return given ? refresh_entries(s, given) : TITAN_GB300_OK;
     // type changes within passive or within active keep the slab order, but
     // the type bits live in the entry words
     if (type) {
@@ -2246,14 +2320,10 @@ int titan_gb300_diagnostics(titan_gb300_sim *s, double g_mag, double energy[4], 
         if (!(s->d_partials = (double *)s->mem.get(tg::kDiagBlocks * tg::kDiagQ * 8, e)))
             return s->cuda_fail(e, "diag alloc");
         if (!(s->d_dout = (double *)s->mem.get(tg::kDiagQ * 8, e))) return s->cuda_fail(e, "diag alloc");
-        if (!(s->d_sk = (double *)s->mem.get(std::max<int64_t>(1, s->ns) * 8, e))) return s->cuda_fail(e, "diag alloc");
-        if (!(s->d_srest = (double *)s->mem.get(std::max<int64_t>(1, s->ns) * 8, e)))
-            return s->cuda_fail(e, "diag alloc");
     }
-    if (s->ns > 0) {
-        CK(cudaMemcpyAsync(s->d_sk, s->k.data(), s->ns * 8, cudaMemcpyHostToDevice, s->stream), "diag upload");
-        CK(cudaMemcpyAsync(s->d_srest, s->rest.data(), s->ns * 8, cudaMemcpyHostToDevice, s->stream), "diag upload");
-    }
+    // (the host arrays change only after a wait for this stream)
+    if (int rc = upload_spring_array(s, titan_gb300_sim::SP_K, s->k)) return rc;
+    if (int rc = upload_spring_array(s, titan_gb300_sim::SP_REST, s->rest)) return rc;
     tg::DiagArgs d{};
     d.state = s->parity ? s->args.state1 : s->args.state0;
     d.mass = s->args.mass;
@@ -2261,8 +2331,8 @@ int titan_gb300_diagnostics(titan_gb300_sim *s, double g_mag, double energy[4], 
     d.npad = s->npad;
     d.sl = s->d_sl;
     d.sr = s->d_sr;
-    d.sk = s->d_sk;
-    d.srest = s->d_srest;
+    d.sk = s->d_sp[titan_gb300_sim::SP_K];
+    d.srest = s->d_sp[titan_gb300_sim::SP_REST];
     d.ns = s->ns;
     d.g_mag = g_mag;
     d.partials = s->d_partials;

@@ -185,8 +185,19 @@ struct XferArgs {
     void *state1;
     void *acc;
     int parity;
-    double *pos, *vel, *accout;  // gather outputs (3*count), any may be null
+    double *pos, *vel, *accout;  // gather outputs (3*count, device or page-locked host), any may be null
+    const int *err;              // the handle's error flag, copied to err_out (page-locked host) if that is given
+    int *err_out;
     const double *ipos, *ivel;   // scatter inputs (3*count), any may be null
+};
+
+// Slab records rewritten from per-spring parameters (creation order): k,
+// rest, damping, omega, amp, phase; a null array leaves its fields.
+struct EntryArgs {
+    const int32_t *spring;  // of each entry
+    void *rec, *act;
+    int64_t count;
+    const double *par[6];
 };
 
 struct DiagArgs {
@@ -277,6 +288,7 @@ cudaError_t launch_gather(int precision, const XferArgs &a, cudaStream_t s);
 cudaError_t launch_export_f32(int precision, const XferArgs &a, float *out, cudaStream_t s);
 cudaError_t launch_scatter(int precision, const XferArgs &a, cudaStream_t s);
 cudaError_t launch_diag(int precision, const DiagArgs &a, cudaStream_t s);
+cudaError_t launch_entries(int precision, const EntryArgs &a, cudaStream_t s);
 
 // A started scene handed to the request server (server.cu): its step
 // arguments and step parity.  serve_begin checks that the server can step

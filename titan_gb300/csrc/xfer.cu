@@ -12,26 +12,42 @@ namespace tg {
 namespace {
 
 // ------------------------------------------------- gather / scatter -------
+// The outputs may be page-locked host memory: a block collects its 256 masses'
+// triples in shared memory and writes them as consecutive doubles, so that a
+// read of a small scene is this one kernel (a copy per array and one for the
+// error flag took 55 us a call, this 25) and a large one moves at the link's
+// rate while it gathers.
+constexpr int kGatherBlock = 256;
 template <int PREC>
-__global__ void k_gather(XferArgs a) {
+__global__ void __launch_bounds__(kGatherBlock) k_gather(XferArgs a) {
     using R = typename Real<PREC>::T;
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.count) return;
-    int64_t src = a.idx ? a.idx[i] : i;
-    int64_t g = a.old2new[src];
-    const St<PREC> s = load_state<PREC>(a.parity ? a.state1 : a.state0, g);
-    const int64_t np = a.npad;
+    __shared__ double buf[3][3 * kGatherBlock];
+    const int64_t i0 = (int64_t)blockIdx.x * kGatherBlock, i = i0 + threadIdx.x;
+    const int t = threadIdx.x;
+    if (i == 0 && a.err_out) *a.err_out = *a.err;
+    if (i < a.count) {
+        const int64_t g = a.old2new[a.idx ? a.idx[i] : i];
+        const St<PREC> s = load_state<PREC>(a.parity ? a.state1 : a.state0, g);
+        const int64_t np = a.npad;
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-        double x = (double)s.x[c], v = (double)s.v[c];
-        if constexpr (PREC == P_FP32C) {
-            x += (double)s.xl[c];
-            v += (double)s.vl[c];
+        for (int c = 0; c < 3; c++) {
+            double x = (double)s.x[c], v = (double)s.v[c];
+            if constexpr (PREC == P_FP32C) {
+                x += (double)s.xl[c];
+                v += (double)s.vl[c];
+            }
+            buf[0][3 * t + c] = x;
+            buf[1][3 * t + c] = v;
+            if (a.accout) buf[2][3 * t + c] = (double)reinterpret_cast<const R *>(a.acc)[c * np + g];
         }
-        if (a.pos) a.pos[3 * i + c] = x;
-        if (a.vel) a.vel[3 * i + c] = v;
-        if (a.accout) a.accout[3 * i + c] = (double)reinterpret_cast<const R *>(a.acc)[c * np + g];
     }
+    __syncthreads();
+    const int m = (int)(a.count - i0 < kGatherBlock ? a.count - i0 : kGatherBlock);
+    double *const out[3] = {a.pos, a.vel, a.accout};
+#pragma unroll
+    for (int w = 0; w < 3; w++)
+        if (out[w])
+            for (int e = t; e < 3 * m; e += kGatherBlock) out[w][3 * i0 + e] = buf[w][e];
 }
 
 // Positions of all masses in caller (creation) order as float triples, the
@@ -80,9 +96,45 @@ __global__ void k_scatter(XferArgs a) {
     store_state<PREC>(a.state1, g, s);
 }
 
+// ------------------------------------------------- entry records ----------
+// One thread per slab entry: the fields of its record and actuation record
+// whose parameters are given, with the host's conversions (upload_records in
+// capi.cu).  Bound by the gathers of 8-byte parameters (a tile's entries are
+// near in creation order) and the strided stores.
+template <int PREC>
+__global__ void __launch_bounds__(256) k_entries(EntryArgs a) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= a.count) return;
+    const int32_t j = a.spring[e];
+    if (j < 0) return;
+    if constexpr (PREC == P_FP64) {
+        double *rec = reinterpret_cast<double *>(a.rec) + 4 * e, *act = reinterpret_cast<double *>(a.act) + 4 * e;
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            if (a.par[q]) rec[q] = a.par[q][j];
+            if (a.par[3 + q]) act[q] = a.par[3 + q][j];
+        }
+    } else {
+        float *rec = reinterpret_cast<float *>(a.rec) + 4 * e, *act = reinterpret_cast<float *>(a.act) + 4 * e;
+        constexpr double kTwoPi = 6.283185307179586476925286766559;
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+            if (a.par[q]) rec[1 + q] = (float)a.par[q][j];
+        if (a.par[1]) act[3] = (float)a.par[1][j];
+        if (a.par[3]) act[0] = (float)(a.par[3][j] / kTwoPi);
+        if (a.par[4]) {
+            const uint32_t type = __float_as_uint(rec[0]) >> 24 & 3u;
+            act[1] = (float)(type == 2 ? -a.par[4][j] : a.par[4][j]);
+        }
+        if (a.par[5]) act[2] = (float)(a.par[5][j] / kTwoPi);
+    }
+}
+
 // ------------------------------------------------------ diagnostics -------
 // Pass 1: each of kDiagBlocks blocks sums a fixed grid-stride share in FP64
 // and reduces it with a fixed tree; pass 2 reduces the partials the same way.
+// The lengths' products and square roots are on the integer units
+// (fp64_alu.cuh).
 template <int PREC>
 __global__ void __launch_bounds__(256) k_diag1(DiagArgs a) {
     __shared__ double red[kDiagQ][256];
@@ -107,7 +159,7 @@ __global__ void __launch_bounds__(256) k_diag1(DiagArgs a) {
         double m = (double)ms[g];
         double x[3] = {pos(s, 0), pos(s, 1), pos(s, 2)};
         double v[3] = {vel(s, 0), vel(s, 1), vel(s, 2)};
-        double vn = nrm3(v[0], v[1], v[2]);
+        double vn = nrm3_alu(v[0], v[1], v[2]);
         q[1] += (0.5 * m) * (vn * vn);
         q[2] += (a.g_mag * x[2]) * m;
         double p[3] = {v[0] * m, v[1] * m, v[2] * m};
@@ -123,7 +175,7 @@ __global__ void __launch_bounds__(256) k_diag1(DiagArgs a) {
         if (l < 0) continue;
         const St<PREC> sl = load_state<PREC>(a.state, l), sr = load_state<PREC>(a.state, r);
         double d0 = pos(sl, 0) - pos(sr, 0), d1 = pos(sl, 1) - pos(sr, 1), d2 = pos(sl, 2) - pos(sr, 2);
-        double x = nrm3(d0, d1, d2) - a.srest[s];
+        double x = nrm3_alu(d0, d1, d2) - a.srest[s];
         q[0] += (a.sk[s] * (x * x)) / 2;
     }
 #pragma unroll
@@ -169,11 +221,11 @@ cudaError_t launch_export_f32(int precision, const XferArgs &a, float *out, cuda
 
 cudaError_t launch_gather(int precision, const XferArgs &a, cudaStream_t s) {
     if (a.count <= 0) return cudaSuccess;
-    int blocks = (int)((a.count + 255) / 256);
+    const int blocks = (int)((a.count + kGatherBlock - 1) / kGatherBlock);
     switch (precision) {
-        case P_FP64: k_gather<P_FP64><<<blocks, 256, 0, s>>>(a); break;
-        case P_FP32: k_gather<P_FP32><<<blocks, 256, 0, s>>>(a); break;
-        default: k_gather<P_FP32C><<<blocks, 256, 0, s>>>(a); break;
+        case P_FP64: k_gather<P_FP64><<<blocks, kGatherBlock, 0, s>>>(a); break;
+        case P_FP32: k_gather<P_FP32><<<blocks, kGatherBlock, 0, s>>>(a); break;
+        default: k_gather<P_FP32C><<<blocks, kGatherBlock, 0, s>>>(a); break;
     }
     return cudaGetLastError();
 }
@@ -185,6 +237,17 @@ cudaError_t launch_scatter(int precision, const XferArgs &a, cudaStream_t s) {
         case P_FP64: k_scatter<P_FP64><<<blocks, 256, 0, s>>>(a); break;
         case P_FP32: k_scatter<P_FP32><<<blocks, 256, 0, s>>>(a); break;
         default: k_scatter<P_FP32C><<<blocks, 256, 0, s>>>(a); break;
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_entries(int precision, const EntryArgs &a, cudaStream_t s) {
+    if (a.count <= 0) return cudaSuccess;
+    const unsigned blocks = (unsigned)((a.count + 255) / 256);
+    switch (precision) {
+        case P_FP64: k_entries<P_FP64><<<blocks, 256, 0, s>>>(a); break;
+        case P_FP32: k_entries<P_FP32><<<blocks, 256, 0, s>>>(a); break;
+        default: k_entries<P_FP32C><<<blocks, 256, 0, s>>>(a); break;
     }
     return cudaGetLastError();
 }
