@@ -94,6 +94,8 @@ def test_heavy_mass_and_uneven_bodies(prec):
     _, ref = run(sc, prec, (0, 0, 0))
     same(st, ref)
     sc = wl.robot_batch(24, side_range=(2, 9))  # some bodies are one tile (no halo), others several
+    sc["pos"][:, 2] -= 0.06  # into their ground planes
+    sc["vel"] = np.random.default_rng(1).normal(scale=0.2, size=sc["pos"].shape)
     _, st = run(sc, prec, None)
     _, ref = run(sc, prec, (0, 0, 0))
     same(st, ref)

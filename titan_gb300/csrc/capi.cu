@@ -1126,6 +1126,7 @@ int build_device(titan_gb300_sim *s) {
                   choose_grid(s, tiles, s->grid_shape, s->gargs.stage, s->grid_smem);
     if (s->use_grid) {
         s->gargs.ntiles = (int32_t)tiles.size();
+        s->gargs.max_nm = P.max_nm;
         std::vector<int32_t> halo(P.halo);
         std::vector<uint8_t> exported(np, 0);
         for (int32_t &h : halo) {

@@ -171,7 +171,7 @@ struct GridResArgs {
     int64_t xbytes;
     uint32_t base;              // passes done since start (tags are base + pass, counts wrap)
     double T0;                  // T of the launch's first step
-    int32_t ntiles;
+    int32_t ntiles, max_nm;     // tiles, and the most masses of one
     int32_t stage;              // 1: slab, actuation and incidence records in shared memory
 };
 

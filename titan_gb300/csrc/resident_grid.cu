@@ -33,6 +33,7 @@
 
 #include "engine.h"
 #include "epilogue.cuh"
+#include "epilogue_lanes.cuh"
 #include "state.cuh"
 #include "step_math.cuh"
 #include "tile_phases.cuh"
@@ -46,6 +47,7 @@ struct GridShape {
     int threads, ctas;
 };
 constexpr GridShape kShapes[kGridShapes] = {{512, 1}, {256, 2}, {128, 4}};
+constexpr int kLaneWarps = 8;  // warps a tile's masses may take with a lane per component
 constexpr uint32_t kGridSpins = 1u << 23;  // polls of one wait: seconds
 
 __host__ __device__ constexpr int64_t rg_align16(int64_t x) { return (x + 15) & ~int64_t(15); }
@@ -113,7 +115,7 @@ __device__ __forceinline__ void record_words(const St<PREC> &s, uint32_t *w) {
     }
 }
 
-template <int PREC, int INTEG, int STAGE, int SHAPE>
+template <int PREC, int INTEG, int STAGE, int SHAPE, bool LANES>
 __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
     k_grid_resident(StepArgs a, GridResArgs r, int parity, int64_t nsteps, int write_acc) {
     using R = typename Real<PREC>::T;
@@ -171,21 +173,26 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
         m = __ldg(reinterpret_cast<const R *>(a.mass) + g_own);
         woff = __ldg(a.warp_inc_off + ti.warp_off + (i_own >> 5)) - inc_base;
     }
-    // FP64: the sum of component c of mass ic, in the warp that has it, where
-    // there is a thread for each (step_kernel.cuh)
+    // FP64: the sum of component c of mass ic, in the thread that has it: on
+    // small tiles a lane per component for the whole mass phase
+    // (epilogue_lanes.cuh), else whole warps per component where there is a
+    // thread for each (step_kernel.cuh)
     const int nmp = (nm + 31) & ~31;
-    const bool split = PREC == P_FP64 && 3 * nmp <= (int)blockDim.x;
-    const int c_sp = (int)threadIdx.x >= 2 * nmp ? 2 : ((int)threadIdx.x >= nmp ? 1 : 0);
-    const int i_sp = (int)threadIdx.x - c_sp * nmp;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool split = PREC == P_FP64 && (LANES || 3 * nmp <= (int)blockDim.x);
+    const int c_sp = LANES ? min(lane / kLaneMasses, 2)
+                           : ((int)threadIdx.x >= 2 * nmp ? 2 : ((int)threadIdx.x >= nmp ? 1 : 0));
+    const int i_sp = !LANES ? (int)threadIdx.x - c_sp * nmp
+                            : lane < 3 * kLaneMasses ? warp * kLaneMasses + lane % kLaneMasses : nm;
     uint32_t d_sp = 0, woff_sp = 0;
     if (split && i_sp < nm) {
         d_sp = __ldg(a.deg + ti.mass_off + i_sp);
-        if (d_sp == 255) d_sp = 0;
+        if (d_sp == 255) d_sp = LANES ? 255 : 0;
         woff_sp = __ldg(a.warp_inc_off + ti.warp_off + (i_sp >> 5)) - inc_base;
     }
 
     // the thread's incidence words
-    const uint32_t d_c = split ? d_sp : (d == 255 ? 0 : d), nw = (d_c + 3) >> 2, pad = (uint32_t)E * 0x10001u;
+    const uint32_t d_c = split ? (d_sp == 255 ? 0 : d_sp) : (d == 255 ? 0 : d), nw = (d_c + 3) >> 2, pad = (uint32_t)E * 0x10001u;
     const uint2 *const ip = reinterpret_cast<const uint2 *>(incb + (split ? woff_sp : woff)) +
                             ((split ? i_sp : i_own) & 31);
     auto word = [&](uint32_t w) { return w >= nw ? make_uint2(pad, pad) : STAGE ? ip[32 * w] : __ldg(ip + 32 * w); };
@@ -200,6 +207,29 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
 #pragma unroll
         for (int c = 0; c < 3; c++) acc0[c] = reinterpret_cast<const R *>(a.acc)[c * np + g_own];
     }
+    LaneMass lm{};
+    double lx = 0.0, lv = 0.0;  // the lane's position and velocity
+    if constexpr (LANES) {
+        lm.c = c_sp;
+        lm.j = lane % kLaneMasses;
+        lm.g = (int64_t)ti.mass_off + i_sp;
+        lm.m = 1.0;
+        if (i_sp < nm) {
+            lm.fl = __ldg(a.flags + lm.g);
+            lm.on = !(lm.fl & MF_FIXED);
+            lm.m = (double)__ldg(reinterpret_cast<const R *>(a.mass) + lm.g);
+            const double *q = reinterpret_cast<const double *>(parity ? a.state1 : a.state0) + 6 * lm.g;
+            lx = q[c_sp];
+            lv = q[3 + c_sp];
+            if (INTEG == INTEG_VERLET) lm.acc0 = reinterpret_cast<const double *>(a.acc)[c_sp * np + lm.g];
+        }
+        lm.gm = a.prm->g[c_sp] * lm.m;
+        uint32_t bad = 0;
+        const Alu y = alu_unpack(lm.m, bad);
+        lm.md = alu_divisor(y);
+        lm.md_ok = !alu_bad(bad) && alu_nonzero(y);
+    }
+    const bool lane_exported = LANES && lm.on && __ldg(r.exported + lm.g) != 0;
     const int64_t passes = nsteps * kPasses;
     for (int64_t pass = 0; pass < passes; pass++) {
         // ---- A: the halo's records of the pass before ------------------------
@@ -281,11 +311,50 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
             heavy_sums<PREC>(a, ti, slots, sH, threadIdx.x >> 5, blockDim.x >> 5);
             __syncthreads();
         }
-            if (split) {
-            if (i_sp < nm) {
-                const double F = gather_list_component(slots, nw, word, c_sp);
-                sF[c_sp * nm + i_sp] = F;
+        if constexpr (LANES) {
+            if (warp * kLaneMasses < nm) {
+                double F = 0;
+                if (d_sp == 255) {
+                    int h = 0;
+                    while (h < ti.nheavy && a.heavy_local[ti.heavy_off + h] != i_sp) h++;
+                    F = F + (double)sH[c_sp * ti.nheavy + h];
+                } else if (i_sp < nm) {
+                    F = gather_list_component(slots, nw, word, c_sp);
+                }
+                __syncwarp();
+                integrate_lanes<INTEG>(a, ti, prm, lm, F, lx, lv, write_acc && pass == passes - 1,
+                                       INTEG == INTEG_RK2 ? (int)(pass & 1) : 0);
+                if (lm.on) {
+                    double *q = reinterpret_cast<double *>(st + (int64_t)i_sp * kRec);
+                    q[c_sp] = lx;
+                    q[3 + c_sp] = lv;
+                    if (pass == passes - 1) {
+                        double *o = reinterpret_cast<double *>((parity ^ (int)(passes & 1)) ? a.state1 : a.state0) + 6 * lm.g;
+                        o[c_sp] = lx;
+                        o[3 + c_sp] = lv;
+                    }
+                }
+                __syncwarp();
+                if (pass < passes - 1) {
+                    // the warp's records to the exchange, a chunk per lane
+                    const uint32_t tag = r.base + (uint32_t)pass + 1;
+                    const uint32_t ex = __ballot_sync(0xffffffffu, lane_exported);
+                    for (int q = lane; q < kLaneMasses * kChunks; q += 32) {
+                        const int k = q / kChunks, c = q % kChunks, i = warp * kLaneMasses + k;
+                        if (!(ex >> k & 1)) continue;  // lane k has mass k's first component
+                        const uint32_t *w = reinterpret_cast<const uint32_t *>(st + (int64_t)i * kRec) + 3 * c;
+                        st_chunk(r.xbuf + (int64_t)((pass + 1) & 1) * r.xbytes +
+                                     (((int64_t)ti.mass_off + i) * kChunks + c) * 16,
+                                 Chunk{{w[0], w[1], w[2]}, tag});
+                    }
+                }
             }
+            Tbefore = T;
+            T = T + prm->launch_dt;
+            continue;
+        }
+        if (split) {
+            if (i_sp < nm) sF[c_sp * nm + i_sp] = gather_list_component(slots, nw, word, c_sp);
             __syncthreads();
         }
         if (!(fl & MF_FIXED)) {  // src/sim.cu:1100
@@ -329,27 +398,35 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
     }
 }
 
-template <int PREC, int INTEG>
+template <int PREC, int INTEG, bool LANES>
 const void *rg_kernel(int stage, int shape) {
     static const void *const f[2][kGridShapes] = {
-        {(const void *)k_grid_resident<PREC, INTEG, 0, 0>, (const void *)k_grid_resident<PREC, INTEG, 0, 1>,
-         (const void *)k_grid_resident<PREC, INTEG, 0, 2>},
-        {(const void *)k_grid_resident<PREC, INTEG, 1, 0>, (const void *)k_grid_resident<PREC, INTEG, 1, 1>,
-         (const void *)k_grid_resident<PREC, INTEG, 1, 2>}};
+        {(const void *)k_grid_resident<PREC, INTEG, 0, 0, LANES>, (const void *)k_grid_resident<PREC, INTEG, 0, 1, LANES>,
+         (const void *)k_grid_resident<PREC, INTEG, 0, 2, LANES>},
+        {(const void *)k_grid_resident<PREC, INTEG, 1, 0, LANES>, (const void *)k_grid_resident<PREC, INTEG, 1, 1, LANES>,
+         (const void *)k_grid_resident<PREC, INTEG, 1, 2, LANES>}};
     return f[stage][shape];
 }
-template <int PREC>
+template <int PREC, bool LANES>
 const void *rg_kernel(int integ, int stage, int shape) {
     switch (integ) {
-        case INTEG_VERLET: return rg_kernel<PREC, INTEG_VERLET>(stage, shape);
-        case INTEG_RK2: return rg_kernel<PREC, INTEG_RK2>(stage, shape);
-        default: return rg_kernel<PREC, INTEG_EULER>(stage, shape);
+        case INTEG_VERLET: return rg_kernel<PREC, INTEG_VERLET, LANES>(stage, shape);
+        case INTEG_RK2: return rg_kernel<PREC, INTEG_RK2, LANES>(stage, shape);
+        default: return rg_kernel<PREC, INTEG_EULER, LANES>(stage, shape);
     }
 }
-const void *rg_kernel(int precision, int integ, int stage, int shape) {
-    return precision == P_FP64   ? rg_kernel<P_FP64>(integ, stage, shape)
-           : precision == P_FP32 ? rg_kernel<P_FP32>(integ, stage, shape)
-                                 : rg_kernel<P_FP32C>(integ, stage, shape);
+// max_nm: the largest tile's masses.  A lane per component serves FP64 tiles
+// of at most kLaneWarps warps of masses (20^3 lattice, 53 masses: 12.5 us per
+// step against 12.9; 24^3, 91 masses: equal, with spills against none)
+const void *rg_kernel(int precision, int integ, int stage, int shape, int max_nm) {
+    if (precision == P_FP64) {
+        const int warps = kShapes[shape].threads / 32;
+        return max_nm <= kLaneMasses * (warps < kLaneWarps ? warps : kLaneWarps)
+                   ? rg_kernel<P_FP64, true>(integ, stage, shape)
+                   : rg_kernel<P_FP64, false>(integ, stage, shape);
+    }
+    return precision == P_FP32 ? rg_kernel<P_FP32, false>(integ, stage, shape)
+                               : rg_kernel<P_FP32C, false>(integ, stage, shape);
 }
 
 }  // namespace
@@ -364,7 +441,7 @@ int grid_resident_ctas(int shape) { return kShapes[shape].ctas; }
 
 cudaError_t launch_grid_resident(int precision, int integ, const StepArgs &a, const GridResArgs &r, int shape,
                                  size_t smem, int parity, int64_t nsteps, int write_acc, cudaStream_t s) {
-    const void *f = rg_kernel(precision, integ, r.stage, shape);
+    const void *f = rg_kernel(precision, integ, r.stage, shape, r.max_nm);
     const cudaError_t e = raise_smem_limit(f, smem);
     if (e != cudaSuccess) return e;
     void *args[] = {const_cast<StepArgs *>(&a), const_cast<GridResArgs *>(&r), &parity, &nsteps, &write_acc};
