@@ -125,3 +125,24 @@ def test_state_changes_between_launches_and_two_handles():
         res.append((a.get_state(acc=True, T=True), b.get_state(acc=True, T=True)))
     same(res[0][0], res[1][0])
     same(res[0][1], res[1][1])
+
+
+@pytest.mark.parametrize("sides", [(3, 9), (6, 9)])
+@pytest.mark.parametrize("prec", [tg.FP32, tg.FP32C])
+def test_many_bodies_in_size_groups(prec, sides):
+    """More bodies than two per SM: whole bodies of up to 512 masses run as
+    resident tiles in size groups, larger ones on the per-step kernels beside
+    them.  Where all are above the per-step tile size, a switch to VERLET keeps
+    state and accelerations as between the per-step kernels."""
+    sc = wl.robot_batch(320, side_range=sides, seed=5)
+    sc["vel"] = np.random.default_rng(2).normal(scale=0.2, size=sc["pos"].shape)
+    s, st = run(sc, prec, None)
+    assert s.resident_info()["active"] == 2 and s.resident_info()["cap"] == 512
+    r, ref = run(sc, prec, (0, 0, 0))
+    same(st, ref)
+    if sides[0] < 6:
+        return
+    for x in (s, r):
+        x.set_integrator(tg.VERLET)
+        x.step(4)
+    same(s.get_state(acc=True, T=True), r.get_state(acc=True, T=True))

@@ -58,12 +58,14 @@ struct DevMem {
 
 }  // namespace
 
+constexpr int kRtGroups = 3;  // size groups of resident tiles
+
 struct titan_gb300_sim {
     int device = 0, prec = P_FP64;
     cudaStream_t stream = nullptr;
-    // resident tiles run on side_stream beside the per-step kernels
-    cudaStream_t side_stream = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    // resident tiles run on side streams beside the per-step kernels
+    cudaStream_t side_stream[kRtGroups] = {};
+    cudaEvent_t ev_fork = nullptr, ev_join[kRtGroups] = {};
     std::string err;
 
     // host scene (creation order)
@@ -154,10 +156,14 @@ struct titan_gb300_sim {
     int res_threads = 0, res_ctas = 0;
     // resident tiles (mode 2): halo-free tiles stepped in shared memory
     bool use_rtiles = false;
-    tg::TileResArgs rtargs{};
     std::vector<tg::TileInfo> rtiles;
-    int rt_threads = 0, rt_mpt = 0;
-    size_t rt_smem = 0;
+    struct RtGroup {  // a launch's share of them, with its shape
+        size_t first = 0;
+        tg::TileResArgs args{};
+        int threads = 0, mpt = 0;
+        size_t smem = 0;
+    };
+    std::vector<RtGroup> rt_groups;
     // all tiles at once (resident_grid.cu); the per-step kernels stay ready
     // for single steps
     bool use_grid = false;
@@ -209,12 +215,14 @@ struct titan_gb300_sim {
         if (stream) cudaStreamSynchronize(stream);
         free_device();
         if (stream) cudaStreamDestroy(stream);
-        if (side_stream) {
-            cudaStreamSynchronize(side_stream);
-            cudaStreamDestroy(side_stream);
+        for (cudaStream_t st : side_stream) {
+            if (!st) continue;
+            cudaStreamSynchronize(st);
+            cudaStreamDestroy(st);
         }
         if (ev_fork) cudaEventDestroy(ev_fork);
-        if (ev_join) cudaEventDestroy(ev_join);
+        for (cudaEvent_t ev : ev_join)
+            if (ev) cudaEventDestroy(ev);
     }
 };
 
@@ -640,6 +648,13 @@ tg::PlanInput plan_input(titan_gb300_sim *s, int tile_masses, bool grid = false)
         } else if (ws) {
             in.tile_cap = fit(4.0, 64, kWsDefaultTile);
             in.whole_cap = kWsDefaultTile;
+            // many bodies: whole ones of up to 512 masses run resident
+            // (Euler), a step of 608 bodies of 6^3 masses in 8.9 us against
+            // 16.5 as two tiles each, of 8^3 in 24.8 against 30.7; of 9^3 in
+            // 42.6 either way
+            if (grid_wanted(s) && s->integrator == tg::INTEG_EULER &&
+                (int64_t)s->body_ptr.size() > 2 * (int64_t)sms)
+                in.whole_cap = 512;
         } else {
             in.tile_cap = 256;
         }
@@ -843,8 +858,12 @@ std::string plan_scene(titan_gb300_sim *s, int tile_masses, tg::PlanInput &in) {
     why = tg::build_plan(in, s->plan);
     if (why.empty() && tile_masses == 0 && in.tile_cap == kWsDefaultTile && !pull_wanted(s)) {
         tg::WsLayout W{};
-        ws_stage_layout(s->prec, tile_infos(s->plan), W);
-        if (W.nstages < 2) {
+        std::vector<tg::TileInfo> tiles = tile_infos(s->plan);
+        if (in.whole_cap > kWsDefaultTile)  // whole bodies above the tile size run resident
+            tiles.erase(std::remove_if(tiles.begin(), tiles.end(), [](const tg::TileInfo &ti) { return ti.nh == 0; }),
+                        tiles.end());
+        if (!tiles.empty()) ws_stage_layout(s->prec, tiles, W);
+        if (!tiles.empty() && W.nstages < 2) {
             in = plan_input(s, kWsFallbackTile);
             why = tg::build_plan(in, s->plan);
         }
@@ -971,7 +990,7 @@ int build_device(titan_gb300_sim *s) {
     // when the largest tile's fit and every tile still gets a CTA at once
     s->use_rtiles = false;
     s->rtiles.clear();
-    s->rtargs = tg::TileResArgs{};
+    s->rt_groups.clear();
     std::vector<uint8_t> rt_flag(P.ntiles, 0);
     // automatic: resident tiles for every halo-free tile that fits when the
     // kernel form is automatic (measured on GB300: 2.5x faster than the
@@ -982,46 +1001,57 @@ int build_device(titan_gb300_sim *s) {
     if ((s->res_mode == 2 || rt_auto) && s->integrator == tg::INTEG_EULER) {
         const size_t kMaxSmem = 227 * 1024;
         const int tcap = s->res_threads_req > 0 ? s->res_threads_req : 512;
-        int64_t max_nm = 0, max_ne = 0;
         for (int64_t t = 0; t < P.ntiles; t++) {
             const tg::TileInfo &ti = tiles[t];
             if (ti.nh != 0 || ti.nm > tg::kResMaxMpt * tcap || tg::tile_resident_smem_bytes(s->prec, ti, 0) > kMaxSmem)
                 continue;
             rt_flag[t] = 1;
             s->rtiles.push_back(ti);
-            max_nm = std::max<int64_t>(max_nm, ti.nm);
-            max_ne = std::max<int64_t>(max_ne, ti.ne);
         }
-        if (!s->rtiles.empty()) {
-            int sms = 0, dev = 0;
-            CK(cudaGetDevice(&dev), "device");
-            CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device");
+        // as many as the SMs or more: the largest first, in groups by size
+        // with a launch each, so that small tiles get small CTAs
+        auto group_of = [&](const tg::TileInfo &ti) { return ti.nm > 256 ? 0 : (ti.nm > 128 ? 1 : 2); };
+        const bool many = (int64_t)s->rtiles.size() >= sms_dev && s->res_threads_req == 0;
+        if (many)
+            std::stable_sort(s->rtiles.begin(), s->rtiles.end(),
+                             [](const tg::TileInfo &x, const tg::TileInfo &y) { return x.nm > y.nm; });
+        for (size_t first = 0; first < s->rtiles.size();) {
+            size_t last = first + 1;
+            while (last < s->rtiles.size() && (!many || group_of(s->rtiles[last]) == group_of(s->rtiles[first]))) last++;
+            titan_gb300_sim::RtGroup g;
+            g.first = first;
+            int64_t max_nm = 0, max_ne = 0;
+            size_t sm_st = 0, sm_pl = 0;
+            for (size_t q = first; q < last; q++) {
+                const tg::TileInfo &ti = s->rtiles[q];
+                max_nm = std::max<int64_t>(max_nm, ti.nm);
+                max_ne = std::max<int64_t>(max_ne, ti.ne);
+                sm_st = std::max(sm_st, tg::tile_resident_smem_bytes(s->prec, ti, 1));
+                sm_pl = std::max(sm_pl, tg::tile_resident_smem_bytes(s->prec, ti, 0));
+            }
             // threads: a thread per mass of the largest tile; with fewer tiles
             // than SMs, up to a quarter of its slab entries (phase B) -- in
             // [64, 512] (measured on GB300: one 125-mass tile steps fastest
             // with 288 threads, thousands of them with 128)
-            const int64_t want_t = (int64_t)s->rtiles.size() < sms ? std::max<int64_t>(max_nm, max_ne / 4) : max_nm;
-            s->rt_threads = s->res_threads_req > 0
-                                ? s->res_threads_req
-                                : (int)std::max<int64_t>(64, std::min<int64_t>(512, (want_t + 31) & ~int64_t(31)));
-            s->rt_mpt = (int)((max_nm + s->rt_threads - 1) / s->rt_threads);
-            size_t sm_st = 0, sm_pl = 0;
-            for (const tg::TileInfo &ti : s->rtiles) {
-                sm_st = std::max(sm_st, tg::tile_resident_smem_bytes(s->prec, ti, 1));
-                sm_pl = std::max(sm_pl, tg::tile_resident_smem_bytes(s->prec, ti, 0));
-            }
+            const int64_t want_t = many ? max_nm : std::max<int64_t>(max_nm, max_ne / 4);
+            g.threads = s->res_threads_req > 0
+                            ? s->res_threads_req
+                            : (int)std::max<int64_t>(64, std::min<int64_t>(512, (want_t + 31) & ~int64_t(31)));
+            g.mpt = (int)((max_nm + g.threads - 1) / g.threads);
             int stage = 0;
-            if (sm_st <= kMaxSmem && tg::tile_resident_prepare(s->prec, s->rt_mpt, 1, sm_st) == cudaSuccess) {
-                const int ps = tg::tile_resident_ctas_per_sm(s->prec, s->rt_mpt, 1, s->rt_threads, sm_st);
-                stage = ps > 0 && (int64_t)s->rtiles.size() <= (int64_t)sms * ps;
+            if (sm_st <= kMaxSmem && tg::tile_resident_prepare(s->prec, g.mpt, 1, sm_st) == cudaSuccess) {
+                const int ps = tg::tile_resident_ctas_per_sm(s->prec, g.mpt, 1, g.threads, sm_st);
+                stage = ps > 0 && (int64_t)(last - first) <= (int64_t)sms_dev * ps;
             }
-            s->rt_smem = stage ? sm_st : sm_pl;
-            CK(tg::tile_resident_prepare(s->prec, s->rt_mpt, stage, s->rt_smem), "set resident-tile shared memory");
-            if (tg::tile_resident_ctas_per_sm(s->prec, s->rt_mpt, stage, s->rt_threads, s->rt_smem) <= 0)
+            g.smem = stage ? sm_st : sm_pl;
+            CK(tg::tile_resident_prepare(s->prec, g.mpt, stage, g.smem), "set resident-tile shared memory");
+            if (tg::tile_resident_ctas_per_sm(s->prec, g.mpt, stage, g.threads, g.smem) <= 0)
                 return s->fail(TITAN_GB300_ELIMIT, "resident tiles do not fit one SM");
+            g.args.ntiles = (int32_t)(last - first);
+            g.args.stage = stage;
             s->use_rtiles = true;
-            s->rtargs.ntiles = (int32_t)s->rtiles.size();
-            s->rtargs.stage = stage;
+            s->rt_groups.push_back(g);
+            first = last;
         }
     }
     std::vector<tg::TileInfo> tiles_run;
@@ -1104,7 +1134,11 @@ int build_device(titan_gb300_sim *s) {
         DEVCOPY(a.pull_units, s->pull.units, "upload pull units");
         DEVCOPY(a.pull_ell, s->pull.ell, "upload pull columns");
     }
-    if (s->use_rtiles) DEVCOPY(s->rtargs.tiles, s->rtiles, "upload resident tiles");
+    if (s->use_rtiles) {
+        tg::TileInfo *rt = nullptr;
+        DEVCOPY(rt, s->rtiles, "upload resident tiles");
+        for (auto &g : s->rt_groups) g.args.tiles = rt + g.first;
+    }
     if (s->use_res) {
         tg::ResPlan &R = s->rplan;
         tg::ResArgs &r = s->rargs;
@@ -1171,10 +1205,15 @@ int build_device(titan_gb300_sim *s) {
     if (!(a.acc = s->mem.get(3 * np * rs, e))) return s->cuda_fail(e, "alloc acc");
     if (!(a.tbuf = (double *)s->mem.get(2 * sizeof(double), e))) return s->cuda_fail(e, "alloc time");
     if (s->use_rtiles) {
-        if (!(s->rtargs.t0 = (const double *)s->mem.get(sizeof(double), e))) return s->cuda_fail(e, "alloc time");
-        if (!s->side_stream) CK(cudaStreamCreateWithFlags(&s->side_stream, cudaStreamNonBlocking), "create stream");
+        const double *t0 = (const double *)s->mem.get(sizeof(double), e);
+        if (!t0) return s->cuda_fail(e, "alloc time");
         if (!s->ev_fork) CK(cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming), "create event");
-        if (!s->ev_join) CK(cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming), "create event");
+        for (size_t q = 0; q < s->rt_groups.size(); q++) {
+            s->rt_groups[q].args.t0 = t0;
+            if (!s->side_stream[q])
+                CK(cudaStreamCreateWithFlags(&s->side_stream[q], cudaStreamNonBlocking), "create stream");
+            if (!s->ev_join[q]) CK(cudaEventCreateWithFlags(&s->ev_join[q], cudaEventDisableTiming), "create event");
+        }
     }
     if (!(s->dprm = (tg::DevParams *)s->mem.get(sizeof(tg::DevParams), e))) return s->cuda_fail(e, "alloc params");
     a.prm = s->dprm;
@@ -1465,9 +1504,9 @@ int titan_gb300_kernel_info(const titan_gb300_sim *s, int64_t out[4]) {
     if (!s || !out) return TITAN_GB300_EINVAL;
     if (s->use_rtiles && s->args.ntiles == 0) {
         out[0] = 5;
-        out[1] = s->rtargs.ntiles;
-        out[2] = s->rt_threads;
-        out[3] = (int64_t)s->rt_smem;
+        out[1] = (int64_t)s->rtiles.size();
+        out[2] = s->rt_groups[0].threads;
+        out[3] = (int64_t)s->rt_groups[0].smem;
         return TITAN_GB300_OK;
     }
     out[0] = s->use_pull ? 6 : (s->use_async ? 3 : (s->use_ws ? 4 : 1));
@@ -1509,9 +1548,9 @@ int titan_gb300_resident_info(const titan_gb300_sim *s, int64_t out[8]) {
         out[2] = (int64_t)(std::unique(bodies.begin(), bodies.end()) - bodies.begin());
         out[3] = nm;
         out[4] = cap;
-        out[5] = s->rt_threads;
+        out[5] = s->rt_groups[0].threads;
         out[6] = (int64_t)s->rtiles.size();
-        out[7] = (int64_t)s->rt_smem;
+        out[7] = (int64_t)s->rt_groups[0].smem;
         return TITAN_GB300_OK;
     }
     if (!s->use_res) return TITAN_GB300_OK;
@@ -1756,7 +1795,42 @@ int titan_gb300_set_integrator(titan_gb300_sim *s, int kind) try {
     if (was_res) {  // resident bins and tiles run Euler only: rebuild without them
         int rc = pull_state(s);
         if (rc) return rc;
-        return build_device(s);
+        // a scene whose bodies are all above the per-step kernels' tile size
+        // is resident only because it has many: its state goes over bit for
+        // bit, and its accelerations (VERLET's state), as between the per-step
+        // kernels
+        bool carry = s->use_rtiles && !s->use_res;
+        for (const tg::TileInfo &ti : s->rtiles) carry = carry && ti.nm > kWsDefaultTile && s->prec != P_FP64;
+        void *rec = nullptr;
+        const size_t rb = (size_t)s->n * tg::state_record_bytes(s->prec), ab = 3 * (size_t)s->n * s->rsize();
+        auto xfer = [&]() {
+            tg::XferArgs x{};
+            x.old2new = s->d_old2new;
+            x.count = s->n;
+            x.npad = s->npad;
+            x.state0 = s->args.state0;
+            x.state1 = s->args.state1;
+            x.acc = s->args.acc;
+            x.parity = s->parity;
+            return x;
+        };
+        if (carry) {
+            CK(cudaMalloc(&rec, rb + ab), "carry state");
+            cudaError_t e = tg::launch_carry(s->prec, xfer(), true, rec, (uint8_t *)rec + rb, s->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+            if (e != cudaSuccess) {
+                cudaFree(rec);
+                return s->cuda_fail(e, "carry state");
+            }
+        }
+        rc = build_device(s);
+        if (carry && rc == TITAN_GB300_OK) {
+            cudaError_t e = tg::launch_carry(s->prec, xfer(), false, rec, (uint8_t *)rec + rb, s->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+            if (e != cudaSuccess) rc = s->cuda_fail(e, "carry state");
+        }
+        if (rec) cudaFree(rec);
+        return rc;
     }
     // the kernels of the new integrator need their shared-memory limit
     if (s->use_pull)
@@ -1874,25 +1948,28 @@ int titan_gb300_step(titan_gb300_sim *s, int64_t nsteps) try {
         CK(tg::launch_resident(s->prec, s->args, s->rargs, s->res_ctas, s->res_threads, s->parity, nsteps, 1,
                                s->args.ntiles == 0, s->stream),
            "launch resident bins");
-    bool joined = true;
+    const bool alone = s->args.ntiles == 0;
     if (s->use_rtiles) {
         // the first step's time, copied before per-step kernels advance the record
-        CK(cudaMemcpyAsync(const_cast<double *>(s->rtargs.t0), s->args.tbuf + s->parity, sizeof(double),
+        CK(cudaMemcpyAsync(const_cast<double *>(s->rt_groups[0].args.t0), s->args.tbuf + s->parity, sizeof(double),
                            cudaMemcpyDeviceToDevice, s->stream),
            "launch resident tiles");
-        if (s->args.ntiles == 0) {
-            CK(tg::launch_tile_resident(s->prec, s->args, s->rtargs, s->rt_mpt, s->rt_threads, s->rt_smem,
-                                        s->parity, nsteps, 1, s->stream),
+        // beside the per-step kernels and each other: disjoint masses (the
+        // first group of a scene without per-step tiles needs no side stream)
+        const size_t first = alone ? 1 : 0;
+        if (s->rt_groups.size() > first) CK(cudaEventRecord(s->ev_fork, s->stream), "launch resident tiles");
+        for (size_t q = 0; q < s->rt_groups.size(); q++) {
+            const auto &g = s->rt_groups[q];
+            cudaStream_t st = q < first ? s->stream : s->side_stream[q];
+            if (q >= first) CK(cudaStreamWaitEvent(st, s->ev_fork, 0), "launch resident tiles");
+            CK(tg::launch_tile_resident(s->prec, s->args, g.args, g.mpt, g.threads, g.smem, s->parity, nsteps, 1, st),
                "launch resident tiles");
+            if (q >= first) CK(cudaEventRecord(s->ev_join[q], st), "launch resident tiles");
+        }
+        if (alone) {
+            for (size_t q = first; q < s->rt_groups.size(); q++)
+                CK(cudaStreamWaitEvent(s->stream, s->ev_join[q], 0), "join resident tiles");
             CK(tg::launch_advance_time(s->args, s->parity, nsteps, s->stream), "advance time");
-        } else {  // beside the per-step kernels: disjoint masses
-            CK(cudaEventRecord(s->ev_fork, s->stream), "launch resident tiles");
-            CK(cudaStreamWaitEvent(s->side_stream, s->ev_fork, 0), "launch resident tiles");
-            CK(tg::launch_tile_resident(s->prec, s->args, s->rtargs, s->rt_mpt, s->rt_threads, s->rt_smem,
-                                        s->parity, nsteps, 1, s->side_stream),
-               "launch resident tiles");
-            CK(cudaEventRecord(s->ev_join, s->side_stream), "launch resident tiles");
-            joined = false;
         }
     }
     if (s->args.ntiles == 0) {
@@ -1919,7 +1996,9 @@ int titan_gb300_step(titan_gb300_sim *s, int64_t nsteps) try {
         return TITAN_GB300_OK;
     }();
     // later work on the handle's stream sees the resident tiles' results
-    if (!joined) CK(cudaStreamWaitEvent(s->stream, s->ev_join, 0), "join resident tiles");
+    if (s->use_rtiles)
+        for (size_t q = 0; q < s->rt_groups.size(); q++)
+            CK(cudaStreamWaitEvent(s->stream, s->ev_join[q], 0), "join resident tiles");
     if (rc) return rc;
     advance_clock(s, nsteps);
     return TITAN_GB300_OK;

@@ -289,6 +289,9 @@ cudaError_t launch_export_f32(int precision, const XferArgs &a, float *out, cuda
 cudaError_t launch_scatter(int precision, const XferArgs &a, cudaStream_t s);
 cudaError_t launch_diag(int precision, const DiagArgs &a, cudaStream_t s);
 cudaError_t launch_entries(int precision, const EntryArgs &a, cudaStream_t s);
+// a.count masses' raw records (rec) and accelerations (acc, component-major)
+// to caller order, or from it into both state buffers
+cudaError_t launch_carry(int precision, const XferArgs &a, bool out, void *rec, void *acc, cudaStream_t s);
 
 // A started scene handed to the request server (server.cu): its step
 // arguments and step parity.  serve_begin checks that the server can step

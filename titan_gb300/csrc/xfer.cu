@@ -96,6 +96,27 @@ __global__ void k_scatter(XferArgs a) {
     store_state<PREC>(a.state1, g, s);
 }
 
+// Raw state records and accelerations to (out) or from caller order, bit for
+// bit: a plan's state carried over to another plan of the same masses.
+template <bool OUT>
+__global__ void __launch_bounds__(256) k_carry(XferArgs a, float4 *rec, uint32_t *acc, int vecs, int words) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.count) return;
+    const int64_t g = a.old2new[i];
+    float4 *const s0 = reinterpret_cast<float4 *>(a.state0) + g * vecs, *const s1 = reinterpret_cast<float4 *>(a.state1) + g * vecs;
+    for (int v = 0; v < vecs; v++) {
+        if (OUT) rec[i * vecs + v] = (a.parity ? s1 : s0)[v];
+        else s0[v] = s1[v] = rec[i * vecs + v];
+    }
+    for (int c = 0; c < 3; c++)
+        for (int w = 0; w < words; w++) {
+            uint32_t *const x = reinterpret_cast<uint32_t *>(a.acc) + (c * a.npad + g) * words + w;
+            uint32_t *const y = acc + (c * a.count + i) * words + w;
+            if (OUT) *y = *x;
+            else *x = *y;
+        }
+}
+
 // ------------------------------------------------- entry records ----------
 // One thread per slab entry: the fields of its record and actuation record
 // whose parameters are given, with the host's conversions (upload_records in
@@ -238,6 +259,15 @@ cudaError_t launch_scatter(int precision, const XferArgs &a, cudaStream_t s) {
         case P_FP32: k_scatter<P_FP32><<<blocks, 256, 0, s>>>(a); break;
         default: k_scatter<P_FP32C><<<blocks, 256, 0, s>>>(a); break;
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_carry(int precision, const XferArgs &a, bool out, void *rec, void *acc, cudaStream_t s) {
+    if (a.count <= 0) return cudaSuccess;
+    const unsigned blocks = (unsigned)((a.count + 255) / 256);
+    const int vecs = state_record_bytes(precision) / 16, words = precision == P_FP64 ? 2 : 1;
+    if (out) k_carry<true><<<blocks, 256, 0, s>>>(a, (float4 *)rec, (uint32_t *)acc, vecs, words);
+    else k_carry<false><<<blocks, 256, 0, s>>>(a, (float4 *)rec, (uint32_t *)acc, vecs, words);
     return cudaGetLastError();
 }
 
