@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
     constexpr int kRec = PREC == P_FP32 ? 32 : 48;
     constexpr int kSlot = Slot<PREC>::kBytes;
     constexpr int kPasses = INTEG == INTEG_RK2 ? 2 : 1;
-    constexpr int kBatch = PREC == P_FP64 ? 1 : 4;
+    constexpr int kBatch = PREC == P_FP64 ? 1 : 3;  // slab entries a thread has in flight (measured best)
     constexpr int kChunks = PREC == P_FP32 ? 2 : 4;  // of one record in the exchange
     constexpr int kPoll = 4;                         // chunks a thread has in flight
     extern __shared__ __align__(16) uint8_t smem[];

@@ -194,6 +194,15 @@ __device__ __forceinline__ F3<PREC> spring_force(int sa, int sb, uint32_t type, 
         return spring_force_f64(sa, sb, k, rs, damping, st);
     } else {
         (void)type;
+        // all of both ends' records before the actuation: the loads' latency
+        // then hides behind it (resident grid, 37^3 lattice 8.7 -> 8.1 us,
+        // 16^3 2.85 -> 2.75; the warp-specialised form: no change)
+        constexpr int kV = PREC == P_FP32 ? 2 : 3;  // float4 per state record
+        const float4 *pa = reinterpret_cast<const float4 *>(st) + sa * kV;
+        const float4 *pb = reinterpret_cast<const float4 *>(st) + sb * kV;
+        const float4 a0 = pa[0], a1 = pa[1], b0 = pb[0], b1 = pb[1];
+        float a2x = 0.f, b2x = 0.f;
+        if constexpr (PREC == P_FP32C) a2x = pa[2].x, b2x = pb[2].x;
         float rs = rest;
         if (actuated) {
             const float4 q = act.v;
@@ -201,13 +210,8 @@ __device__ __forceinline__ F3<PREC> spring_force(int sa, int sb, uint32_t type, 
             const float fr = cyc - rintf(cyc);
             rs = rest * fmaf(q.y, __sinf(6.28318530717958647692f * fr), 1.0f);
         }
-        constexpr int kV = PREC == P_FP32 ? 2 : 3;  // float4 per state record
-        const float4 *pa = reinterpret_cast<const float4 *>(st) + sa * kV;
-        const float4 *pb = reinterpret_cast<const float4 *>(st) + sb * kV;
-        const float4 a0 = pa[0], a1 = pa[1], b0 = pb[0], b1 = pb[1];
         float d0 = b0.x - a0.x, d1 = b0.y - a0.y, d2 = b0.z - a0.z;
         if constexpr (PREC == P_FP32C) {
-            const float a2x = pa[2].x, b2x = pb[2].x;
             d0 += b1.z - a1.z;
             d1 += b1.w - a1.w;
             d2 += b2x - a2x;
