@@ -181,7 +181,11 @@ int titan_gb300_set_occupancy(titan_gb300_sim *sim, int min_ctas_per_sm);
 /* Step kernel form (extension; the reference has one pair of kernels):
  * 0 = automatic: the warp-specialised kernel in FP32 and FP32C (measured
  * fastest on GB300), the per-tile kernel in FP64, and resident tiles for
- * halo-free tiles (set_resident); 1 = per-tile kernel (one CTA per tile);
+ * halo-free tiles (set_resident); a step() of two steps or more on a scene
+ * whose tiles all get a CTA at once (about 29,000 masses in FP64, 63,000 in
+ * FP32C) then runs them in one launch that keeps the state on chip, unless
+ * a form, launch shape, register cap or resident mode was chosen;
+ * 1 = per-tile kernel (one CTA per tile);
  * 3 = per-tile kernel whose slab records and tile states arrive by bulk
  * copy (TMA) and halo by cp.async, all issued before one wait; 4 =
  * warp-specialised persistent kernel (a producer warp streams tiles into a
@@ -193,7 +197,8 @@ int titan_gb300_set_occupancy(titan_gb300_sim *sim, int min_ctas_per_sm);
  * start(). */
 int titan_gb300_set_kernel(titan_gb300_sim *sim, int variant);
 
-/* After start(): out[0] kernel form of the per-step launches (1 to 4; 5
+/* After start(): out[0] kernel form of the per-step launches (single steps
+ * and what the one-launch form of set_kernel 0 does not hold) (1 to 4; 5
  * when resident tiles carry the whole scene and no per-step kernel runs),
  * out[1] CTAs per launch, out[2] threads per CTA, out[3] dynamic shared
  * memory per CTA (bytes) -- of the resident-tile launch for form 5. */

@@ -537,9 +537,9 @@ bool grid_wanted(const titan_gb300_sim *s) {
 // The resident grid's launch for these tiles (resident_grid.cu): every tile
 // gets a CTA at once, with the slab in shared memory if that fits.  Small
 // tiles get small CTAs, which leave the SMs to other handles' kernels: FP64
-// 256 threads up to 300 entries, else 512 (9^3: 7.4 us per step with either,
-// 8.3 with 128); the FP32 forms 128 up to 400 entries, else 256 (16^3: 2.85
-// us with 128, 3.1 with 256; 24 scenes of 27 to 60,000 masses in flight
+// 256 threads up to 300 entries, else 512 (9^3, before the mass phase with
+// lanes: 7.4 us per step with either, 8.3 with 128); the FP32 forms 128 up to
+// 400 entries, else 256 (16^3: 2.85 us with 128, 3.1 with 256; 24 scenes of 27 to 60,000 masses in flight
 // together, 200 steps: 8.2 against 10.5 ms).  Returns false when the tiles do
 // not all fit.
 bool choose_grid(const titan_gb300_sim *s, const std::vector<tg::TileInfo> &tiles, int &shape, int &stage, size_t &bytes) {
@@ -574,7 +574,8 @@ bool choose_grid(const titan_gb300_sim *s, const std::vector<tg::TileInfo> &tile
 // forms, where two CTAs fill each other's waits.  Measured, us per step, in
 // FP64 at 1 and 2 tiles per SM: 24^3 18.0 and 19.0, 30^3 28.9 and 31.0; in
 // FP32C 16^3 3.48 and 3.15, 30^3 6.6 and 6.2 -- and with the per-step
-// kernels 22.4, 32.2, 4.1 and 7.9.  At least 8 masses per tile in FP64 (9^3:
+// kernels 22.4, 32.2, 4.1 and 7.9 (all before later steps: now 17.4, 28.0,
+// 2.7 and 5.7 with the sizes chosen here).  At least 8 masses per tile in FP64 (9^3:
 // 7.4 us per step against 8.0 with 16), 16 in the FP32 forms (2.7 against 2.5
 // with 8, but half the CTAs).  Bodies up to whole masses stay one tile.
 // Above 192 masses (FP64) or 208 (FP32C: 63,000 in all) per tile the SM's
@@ -618,7 +619,8 @@ tg::PlanInput plan_input(titan_gb300_sim *s, int tile_masses, bool grid = false)
     in.nbodies = s->body_ptr.empty() ? 0 : (int64_t)s->body_ptr.size() - 1;
     in.body_ptr = s->body_ptr.empty() ? nullptr : s->body_ptr.data();
     // Default tile.  Large scenes: 96 masses in FP64 (three CTAs per SM,
-    // step_var.cu; 256 where a form was chosen), 208 for the FP32 forms' warp-specialised
+    // step_var.cu: 80^3 449 us per step against 496 with 256; 256 where a form
+    // was chosen), 208 for the FP32 forms' warp-specialised
     // kernel (two stages fit one SM's shared memory; 192 where they would
     // not, plan_scene) and 256 for the per-tile forms.  Smaller scenes get
     // smaller tiles so that their tiles cover the SMs: FP64 about 1.6 tiles
@@ -626,10 +628,9 @@ tg::PlanInput plan_input(titan_gb300_sim *s, int tile_masses, bool grid = false)
     // 4 (64 to 208).  In the FP32 forms a body that fits the large-scene
     // tile stays whole (a halo-free tile runs resident: 2.0 us per step for
     // the 5^3 lattice against 3.3 split in four); in FP64, bound by each
-    // SM's FP64 pipe, it is split like the rest (17.9 us in four tiles
-    // against 28.9 resident).  Measured on GB300, 20^3 lattice: FP64 37 us
-    // per step with 32-mass tiles against 90 with 256; FP32C 5.3 us with
-    // 64 against 6.5 with 208.
+    // SM's FP64 pipe, it is split like the rest (5^3: 8.6 us in four tiles).
+    // Measured on GB300, 20^3 lattice, per-step kernels: FP64 16.1 us per
+    // step with 32-mass tiles; FP32C 5.3 us with 64 against 6.5 with 208.
     const bool pull = pull_wanted(s);
     const bool ws = !pull && (s->kernel_req == 0 || s->kernel_req == 4);
     if (tile_masses > 0) {

@@ -20,10 +20,11 @@
 // fixed masses are neither written nor waited for.
 //
 // Measured, us per step, with the per-step kernels and here: FP64 5^3 8.6 ->
-// 5.7, 9^3 12.7 -> 7.4, 20^3 16.1 -> 13.3, 30^3 32.2 -> 28.9, 96 bodies of 3-9
-// masses per side 38.6 -> 26.9; FP32C 9^3 4.0 -> 2.7, 16^3 4.1 -> 2.9, 23^3 5.6
-// -> 4.1, 37^3 11.8 -> 8.7.  The exchange is about 0.7 us of a step; the rest is the
-// latency of one tile's phases.
+// 4.6, 9^3 12.7 -> 6.2, 20^3 16.1 -> 12.3, 24^3 22.4 -> 17.4, 30^3 32.2 -> 28.0,
+// 96 bodies of 3-9 masses per side 38.6 -> 27.0; FP32C 9^3 4.0 -> 2.6, 16^3 4.1
+// -> 2.7, 23^3 5.6 -> 3.9, 30^3 7.9 -> 5.7, 37^3 11.8 -> 8.1.  The exchange is
+// about 0.7 us of a step; the rest is the latency of one tile's phases (20^3
+// FP64: FP64 pipe 46 % busy, 1.55 instructions per clock; 23^3 FP32C: 1.43).
 //
 // The phases and the order of every sum are the per-step kernels'
 // (tile_phases.cuh, epilogue.cuh): the results are the same bits.  Waits are
