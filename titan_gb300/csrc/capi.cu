@@ -537,11 +537,15 @@ bool grid_wanted(const titan_gb300_sim *s) {
 // The resident grid's launch for these tiles (resident_grid.cu): every tile
 // gets a CTA at once, with the slab in shared memory if that fits.  Small
 // tiles get small CTAs, which leave the SMs to other handles' kernels: FP64
-// 256 threads up to 300 entries, else 512 (9^3, before the mass phase with
-// lanes: 7.4 us per step with either, 8.3 with 128); the FP32 forms 128 up to
-// 400 entries, else 256 (16^3: 2.85 us with 128, 3.1 with 256; 24 scenes of 27 to 60,000 masses in flight
-// together, 200 steps: 8.2 against 10.5 ms).  Returns false when the tiles do
-// not all fit.
+// 256 threads up to 600 entries, else 512.  From 300 to 600 entries (2,000 to
+// 4,500 masses) the wider CTA is 10 % faster alone (14^3: 7.4 us per step
+// against 8.2; above, 17^3: 9.6 against 10.4), but it fills the SM, so that
+// scenes in flight together take turns: 4 scenes of 27 to 4,000 masses, 300
+// steps, 6.2 against 3.0 ms, 24 of 27 to 3,000, 190 steps, 12.8 against 9.8.
+// 128 threads: 9^3 7.5 us against 6.2.  The FP32 forms 128 up to 400 entries,
+// else 256 (16^3: 2.85 us with 128, 3.1 with 256; 24 scenes of 27 to 60,000
+// masses in flight together, 200 steps: 8.2 against 10.5 ms).  Returns false
+// when the tiles do not all fit.
 bool choose_grid(const titan_gb300_sim *s, const std::vector<tg::TileInfo> &tiles, int &shape, int &stage, size_t &bytes) {
     size_t smem[2] = {0, 0};
     int max_nm = 0, max_ne = 0;
@@ -551,7 +555,7 @@ bool choose_grid(const titan_gb300_sim *s, const std::vector<tg::TileInfo> &tile
         for (int st = 0; st < 2; st++) smem[st] = std::max(smem[st], tg::grid_resident_smem_bytes(s->prec, ti, st));
     }
     int first;
-    if (s->prec == P_FP64) first = max_ne <= 300 ? 1 : 0;
+    if (s->prec == P_FP64) first = max_ne <= 600 ? 1 : 0;
     else first = max_ne <= 400 ? 2 : 1;
     const int order[3][tg::kGridShapes] = {{0, 1, 2}, {1, 0, 2}, {2, 1, 0}};
     for (const int sh : order[first]) {
