@@ -183,7 +183,7 @@ int titan_gb300_set_occupancy(titan_gb300_sim *sim, int min_ctas_per_sm);
  * fastest on GB300), the per-tile kernel in FP64, and resident tiles for
  * halo-free tiles (set_resident); a step() of two steps or more on a scene
  * whose tiles all get a CTA at once (about 29,000 masses in FP64, 63,000 in
- * FP32C) then runs them in one launch that keeps the state on chip, unless
+ * FP32C) then runs up to 512 at a time in one launch that keeps the state on chip, unless
  * a form, launch shape, register cap or resident mode was chosen;
  * 1 = per-tile kernel (one CTA per tile);
  * 3 = per-tile kernel whose slab records and tile states arrive by bulk

@@ -146,3 +146,19 @@ def test_many_bodies_in_size_groups(prec, sides):
         x.set_integrator(tg.VERLET)
         x.step(4)
     same(s.get_state(acc=True, T=True), r.get_state(acc=True, T=True))
+
+
+@pytest.mark.parametrize("integ", [tg.EULER, tg.VERLET, tg.RK2])
+@pytest.mark.parametrize("prec", [tg.FP64, tg.FP32C])
+def test_long_calls_in_several_launches(prec, integ):
+    """Calls on both sides of the launches' 512 steps, and odd remainders."""
+    sc = scene(6, 7, 8, seed=4, fixed=0.05, act=0.2 if prec != tg.FP64 else 0.0)
+    sc["integrator"] = integ
+    got = []
+    for resident in (None, (0, 0, 0)):
+        s = wl.make_sim(sc, prec, resident=resident)
+        for n in (512, 513, 1027):
+            s.step(n)
+        got.append(s.get_state(acc=True, T=True))
+    assert np.isfinite(got[1]["pos"]).all()
+    same(*got)

@@ -503,6 +503,12 @@ constexpr bool kPullAuto = false;
 constexpr int kHeavyThreshold = 96;
 constexpr int64_t kGridMinSteps = 2;
 
+// Steps of one resident-grid launch: other handles' kernels get no SM that its
+// CTAs fill until it ends, so long calls are cut (100 steps of a 24^3 scene
+// beside 200,000 of a 9^3 one, FP64: 5 ms; in one launch 1.39 s, to that one's
+// end).  A launch costs about 6 us more than its steps, 0.1 to 0.4 % of 512.
+constexpr int64_t kGridMaxSteps = 512;
+
 // Whether the step will run the pull form: when requested (set_kernel 6).
 // (It needs a plan without heavy masses: it has no warp-cooperative sums.)
 bool pull_wanted(const titan_gb300_sim *s) {
@@ -1935,19 +1941,24 @@ int titan_gb300_step(titan_gb300_sim *s, int64_t nsteps) try {
     if (!ensure_device(s)) return s->fail(TITAN_GB300_ECUDA, "cudaSetDevice failed");
     cudaError_t e = cudaSuccess;
     if (grid_runs(s, nsteps)) {
-        s->gargs.T0 = s->T;
-        const cudaError_t r = tg::launch_grid_resident(s->prec, s->integrator, s->args, s->gargs, s->grid_shape,
-                                                       s->grid_smem, s->parity, nsteps, 1, s->stream);
-        if (r == cudaSuccess) {
-            const int P = s->passes();
-            s->gargs.base += (uint32_t)(nsteps * P);
-            s->parity ^= (int)((nsteps * P) & 1);
-            advance_clock(s, nsteps);
-            return TITAN_GB300_OK;
+        while (nsteps > 0 && s->use_grid) {
+            const int64_t len = std::min(nsteps, kGridMaxSteps);
+            s->gargs.T0 = s->T;
+            const cudaError_t r = tg::launch_grid_resident(s->prec, s->integrator, s->args, s->gargs, s->grid_shape,
+                                                           s->grid_smem, s->parity, len, 1, s->stream);
+            if (r == cudaSuccess) {
+                const int P = s->passes();
+                s->gargs.base += (uint32_t)(len * P);
+                s->parity ^= (int)((len * P) & 1);
+                advance_clock(s, len);
+                nsteps -= len;
+                continue;
+            }
+            if (r != cudaErrorCooperativeLaunchTooLarge) return s->cuda_fail(r, "launch resident grid");
+            cudaGetLastError();
+            s->use_grid = false;  // the device has less room than planned for: per-step kernels
         }
-        if (r != cudaErrorCooperativeLaunchTooLarge) return s->cuda_fail(r, "launch resident grid");
-        cudaGetLastError();
-        s->use_grid = false;  // the device has less room than planned for: per-step kernels
+        if (nsteps == 0) return TITAN_GB300_OK;
     }
     if (s->use_res)
         CK(tg::launch_resident(s->prec, s->args, s->rargs, s->res_ctas, s->res_threads, s->parity, nsteps, 1,

@@ -1,5 +1,5 @@
 // resident_grid.cu -- every tile of a scene on its own CTA, all steps of a
-// call in one cooperative launch.
+// call in one cooperative launch (calls above 512 steps in several).
 //
 // The per-step kernels pay, for every step, a launch, the staging of each
 // tile's state and slab, and the drain at the grid's end; on a scene whose
