@@ -545,7 +545,8 @@ bool grid_wanted(const titan_gb300_sim *s) {
 // tiles get small CTAs, which leave the SMs to other handles' kernels: FP64
 // 256 threads up to 600 entries, else 512.  From 300 to 600 entries (2,000 to
 // 4,500 masses) the wider CTA is 10 % faster alone (14^3: 7.4 us per step
-// against 8.2; above, 17^3: 9.6 against 10.4), but it fills the SM, so that
+// against 8.2; a 61 x 11 x 7 beam with drag and a ball 5 %; above, 17^3: 9.6
+// against 10.4), but it fills the SM, so that
 // scenes in flight together take turns: 4 scenes of 27 to 4,000 masses, 300
 // steps, 6.2 against 3.0 ms, 24 of 27 to 3,000, 190 steps, 12.8 against 9.8.
 // 128 threads: 9^3 7.5 us against 6.2.  The FP32 forms 128 up to 400 entries,
