@@ -1235,6 +1235,7 @@ int build_device(titan_gb300_sim *s) {
     if (!(s->d_xfer = (double *)s->mem.get(9 * (size_t)s->n * 8, e))) return s->cuda_fail(e, "alloc staging");
     if (!(s->d_idx = (int64_t *)s->mem.get((size_t)s->n * 8, e))) return s->cuda_fail(e, "alloc staging");
     CK(cudaMallocHost(&s->h_xfer, 9 * (size_t)s->n * 8 + 16), "alloc pinned staging");
+    CK(tg::xfer_prepare(s->prec), "load transfer kernels");
     s->h_err = reinterpret_cast<int *>(s->h_xfer + 9 * s->n);
     CK(cudaMemset(a.state0, 0, s->comps() * np * rs), "clear state");
     CK(cudaMemset(a.state1, 0, s->comps() * np * rs), "clear state");

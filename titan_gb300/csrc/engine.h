@@ -283,6 +283,8 @@ int grid_resident_ctas(int shape);
 int grid_resident_exchange_bytes(int precision);
 cudaError_t launch_grid_resident(int precision, int integ, const StepArgs &a, const GridResArgs &r, int shape,
                                  size_t smem, int parity, int64_t nsteps, int write_acc, cudaStream_t s);
+// loads the transfer kernels' code on the current device
+cudaError_t xfer_prepare(int precision);
 cudaError_t launch_gather(int precision, const XferArgs &a, cudaStream_t s);
 // float positions of all a.count masses in caller order into out (device)
 cudaError_t launch_export_f32(int precision, const XferArgs &a, float *out, cudaStream_t s);

@@ -12,42 +12,51 @@ namespace tg {
 namespace {
 
 // ------------------------------------------------- gather / scatter -------
-// The outputs may be page-locked host memory: a block collects its 256 masses'
-// triples in shared memory and writes them as consecutive doubles, so that a
-// read of a small scene is this one kernel (a copy per array and one for the
-// error flag took 55 us a call, this 25) and a large one moves at the link's
-// rate while it gathers.
+// The outputs may be page-locked host memory: a warp exchanges its 32 masses'
+// triples by shuffles and writes them as consecutive doubles, so that a read
+// of a small scene is this one kernel (a copy per array and one for the error
+// flag took 55 us a call, this 25) and a large one moves at the link's rate
+// while it gathers.  No shared memory and few registers: the request loop
+// (server.cu) leaves 6,688 bytes and a quarter of the register file on each
+// SM, and reads of finished scenes have to run beside it.
 constexpr int kGatherBlock = 256;
+__device__ __forceinline__ void store_triples(double *out, int64_t i0, int64_t count, double x0, double x1, double x2) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+        const int e = 32 * r + lane, src = e / 3, c = e - 3 * src;
+        const double y0 = __shfl_sync(0xffffffffu, x0, src), y1 = __shfl_sync(0xffffffffu, x1, src),
+                     y2 = __shfl_sync(0xffffffffu, x2, src);
+        if (i0 + src < count) out[3 * i0 + e] = c == 0 ? y0 : (c == 1 ? y1 : y2);
+    }
+}
 template <int PREC>
 __global__ void __launch_bounds__(kGatherBlock) k_gather(XferArgs a) {
     using R = typename Real<PREC>::T;
-    __shared__ double buf[3][3 * kGatherBlock];
-    const int64_t i0 = (int64_t)blockIdx.x * kGatherBlock, i = i0 + threadIdx.x;
-    const int t = threadIdx.x;
+    const int64_t i = (int64_t)blockIdx.x * kGatherBlock + threadIdx.x, i0 = i - (threadIdx.x & 31);
     if (i == 0 && a.err_out) *a.err_out = *a.err;
-    if (i < a.count) {
-        const int64_t g = a.old2new[a.idx ? a.idx[i] : i];
+    if (i0 >= a.count) return;  // whole warps
+    // lanes past the end repeat the last mass and store nothing
+    const int64_t j = i < a.count ? i : a.count - 1;
+    const int64_t g = a.old2new[a.idx ? a.idx[j] : j];
+    if (a.pos || a.vel) {
         const St<PREC> s = load_state<PREC>(a.parity ? a.state1 : a.state0, g);
-        const int64_t np = a.npad;
+        double x[3], v[3];
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            double x = (double)s.x[c], v = (double)s.v[c];
+            x[c] = (double)s.x[c], v[c] = (double)s.v[c];
             if constexpr (PREC == P_FP32C) {
-                x += (double)s.xl[c];
-                v += (double)s.vl[c];
+                x[c] += (double)s.xl[c];
+                v[c] += (double)s.vl[c];
             }
-            buf[0][3 * t + c] = x;
-            buf[1][3 * t + c] = v;
-            if (a.accout) buf[2][3 * t + c] = (double)reinterpret_cast<const R *>(a.acc)[c * np + g];
         }
+        if (a.pos) store_triples(a.pos, i0, a.count, x[0], x[1], x[2]);
+        if (a.vel) store_triples(a.vel, i0, a.count, v[0], v[1], v[2]);
     }
-    __syncthreads();
-    const int m = (int)(a.count - i0 < kGatherBlock ? a.count - i0 : kGatherBlock);
-    double *const out[3] = {a.pos, a.vel, a.accout};
-#pragma unroll
-    for (int w = 0; w < 3; w++)
-        if (out[w])
-            for (int e = t; e < 3 * m; e += kGatherBlock) out[w][3 * i0 + e] = buf[w][e];
+    if (a.accout) {
+        const R *acc = reinterpret_cast<const R *>(a.acc) + g;
+        store_triples(a.accout, i0, a.count, (double)acc[0], (double)acc[a.npad], (double)acc[2 * a.npad]);
+    }
 }
 
 // Positions of all masses in caller (creation) order as float triples, the
@@ -228,6 +237,24 @@ __global__ void __launch_bounds__(256) k_diag2(DiagArgs a) {
 
 }  // namespace
 
+
+template <int PREC>
+static cudaError_t load_transfers() {
+    const void *const f[] = {(const void *)k_gather<PREC>, (const void *)k_scatter<PREC>,
+                             (const void *)k_export_f32<PREC>, (const void *)k_entries<PREC>};
+    cudaError_t e = cudaSuccess;
+    cudaFuncAttributes at;
+    for (const void *k : f)
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, k);
+    return e;
+}
+// A kernel's first use loads its code, and that waits for running kernels --
+// beside the request loop, until the loop leaves.
+cudaError_t xfer_prepare(int precision) {
+    return precision == P_FP64   ? load_transfers<P_FP64>()
+           : precision == P_FP32 ? load_transfers<P_FP32>()
+                                 : load_transfers<P_FP32C>();
+}
 
 cudaError_t launch_export_f32(int precision, const XferArgs &a, float *out, cudaStream_t s) {
     if (a.count <= 0) return cudaSuccess;
