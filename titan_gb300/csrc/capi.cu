@@ -129,6 +129,9 @@ struct titan_gb300_sim {
     double *d_sp[SP_COUNT] = {};
     bool sp_current[SP_COUNT] = {};
     int32_t *d_espring = nullptr;
+    // a kernel that writes the slab records may still run: the next step
+    // kernel, which reads them before its grid_dep_wait(), must not start early
+    bool tables_written = false;
 
     size_t rsize() const { return prec == P_FP64 ? sizeof(double) : sizeof(float); }
     int comps() const { return tg::state_words(prec); }
@@ -180,7 +183,8 @@ struct titan_gb300_sim {
         if (args.ntiles == 0) return cudaSuccess;
         args.rk2_stage = stage;
         if (use_pull) return tg::launch_step_pull(prec, integrator, args, ctas, parity, write_acc, stream);
-        if (use_ws) return tg::launch_step_ws(prec, integrator, args, ctas, ws_warps, parity, write_acc, stream);
+        if (use_ws)
+            return tg::launch_step_ws(prec, integrator, args, ctas, ws_warps, parity, write_acc, stream, !tables_written);
         if (use_async)
             return tg::launch_step_async(prec, args, (int)args.ntiles, threads, smem, parity, write_acc, stream);
         return tg::launch_step(prec, step_variant, integrator, args, (int)args.ntiles, threads, smem, parity,
@@ -917,6 +921,7 @@ int refresh_entries(titan_gb300_sim *s, unsigned given) {
         x.par[q] = s->d_sp[q];
     }
     CK(tg::launch_entries(s->prec, x, s->stream), "refresh entries");
+    s->tables_written = true;
     return TITAN_GB300_OK;
 }
 
@@ -1334,12 +1339,15 @@ cudaGraphExec_t get_graph(titan_gb300_sim *s, int len, int parity, cudaError_t &
     if (e != cudaSuccess) return nullptr;
     int p = parity;
     cudaError_t el = cudaSuccess;  // the first launch refused while capturing
+    const bool written = s->tables_written;
+    s->tables_written = false;  // the graph's first step starts after all work before it
     for (int i = 0; i < len; i++)
         for (int q = 0; q < s->passes(); q++) {
             const cudaError_t r = s->launch(p, 0, q);
             if (el == cudaSuccess) el = r;
             p ^= 1;
         }
+    s->tables_written = written;
     e = cudaStreamEndCapture(s->stream, &g);
     if (e == cudaSuccess && el != cudaSuccess) {
         cudaGraphDestroy(g);
@@ -2004,11 +2012,13 @@ int titan_gb300_step(titan_gb300_sim *s, int64_t nsteps) try {
             cudaGraphExec_t g = get_graph(s, len, s->parity, e);
             if (!g) return s->cuda_fail(e, "build step graph");
             CK(cudaGraphLaunch(g, s->stream), "launch step graph");
+            s->tables_written = false;
             s->parity ^= ((len * P) & 1);
             rem -= len;
         }
         for (int q = 0; q < P; q++) {  // the last step also writes the accelerations
             CK(s->launch(s->parity, q == P - 1, q), "launch step");
+            s->tables_written = false;
             s->parity ^= 1;
         }
         return TITAN_GB300_OK;

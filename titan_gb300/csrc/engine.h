@@ -242,8 +242,9 @@ cudaError_t launch_step_async(int precision, const StepArgs &a, int ntiles, int 
 // consumer_warps + 1 warps; the last warp streams tiles into a ring of
 // stages, the others compute.
 cudaError_t step_ws_prepare(int precision, int integ, size_t smem);
+// programmatic: may start while the kernel before it on the stream drains
 cudaError_t launch_step_ws(int precision, int integ, const StepArgs &a, int ctas, int consumer_warps, int parity,
-                           int write_acc, cudaStream_t s);
+                           int write_acc, cudaStream_t s, bool programmatic);
 // Pull kernel (step_pull.cu): `ctas` persistent CTAs of a.pull's teams
 // plus a producer warp; FP32 and FP32C only.
 cudaError_t step_pull_prepare(int precision, int integ, size_t smem);

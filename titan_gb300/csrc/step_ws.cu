@@ -338,7 +338,7 @@ cudaError_t step_ws_prepare(int precision, int integ, size_t smem) {
 }
 
 cudaError_t launch_step_ws(int precision, int integ, const StepArgs &a, int ctas, int consumer_warps, int parity,
-                           int write_acc, cudaStream_t s) {
+                           int write_acc, cudaStream_t s, bool programmatic) {
     if (a.ntiles <= 0) return cudaSuccess;
     if (consumer_warps < 2 || consumer_warps > kWsMaxConsumerWarps || (consumer_warps & 1))
         return cudaErrorInvalidValue;
@@ -346,7 +346,7 @@ cudaError_t launch_step_ws(int precision, int integ, const StepArgs &a, int ctas
     // while this one drains (the kernel orders its dependent reads itself)
     void *args[] = {const_cast<StepArgs *>(&a), &parity, &write_acc};
     return launch_programmatic(ws_kernel(precision, integ), dim3(ctas), dim3((consumer_warps + kWsProducerWarps) * 32), args,
-                               (size_t)a.ws.total, s);
+                               (size_t)a.ws.total, s, programmatic);
 }
 
 }  // namespace tg
