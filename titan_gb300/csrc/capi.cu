@@ -7,6 +7,8 @@
 // fused step kernel on a private stream.
 #include "titan_gb300.h"
 
+#include <cuda.h>
+
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -117,6 +119,7 @@ struct titan_gb300_sim {
     double *d_xfer = nullptr;     // 9n doubles
     int64_t *d_idx = nullptr;     // n
     double *h_xfer = nullptr;     // pinned 9n doubles, then the error flag k_gather copies
+    double *stage_dev = nullptr;  // h_xfer's address on the device
     int *h_err = nullptr;
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
     // diagnostics (lazy)
@@ -238,15 +241,38 @@ namespace {
         if (e_ != cudaSuccess) return s->cuda_fail(e_, what); \
     } while (0)
 
-// A page-locked host buffer's address on the device (cudaMallocHost or
-// cudaHostRegister), null for other memory.
-void *host_on_device(const void *p) {
+// A host buffer's address on the device where all its bytes lie in one
+// page-locked range (cudaMallocHost or cudaHostRegister) that the device may
+// write, null for other memory: kernels store there, and a store past the
+// range (an array registered in part) or into a read-only registration would
+// be an illegal access.
+void *host_on_device(const void *p, size_t bytes) {
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
-    return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+    if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
+    using Query = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+    static const Query query = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found{};
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &found) != cudaSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Query>(found == cudaDriverEntryPointSuccess ? f : nullptr);
+    }();
+    const CUdeviceptr d = (CUdeviceptr)at.devicePointer;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    int access = 0;
+    if (!query || query(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, d) != CUDA_SUCCESS ||
+        query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, d) != CUDA_SUCCESS ||
+        query(&access, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS, d) != CUDA_SUCCESS)
+        return nullptr;
+    const bool inside = d >= start && bytes <= size && d - start <= size - bytes;
+    return inside && access == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE ? at.devicePointer : nullptr;
 }
 
 // Whether a caller's host buffer is page-locked (cudaMallocHost or
@@ -1240,6 +1266,7 @@ int build_device(titan_gb300_sim *s) {
     if (!(s->d_xfer = (double *)s->mem.get(9 * (size_t)s->n * 8, e))) return s->cuda_fail(e, "alloc staging");
     if (!(s->d_idx = (int64_t *)s->mem.get((size_t)s->n * 8, e))) return s->cuda_fail(e, "alloc staging");
     CK(cudaMallocHost(&s->h_xfer, 9 * (size_t)s->n * 8 + 16), "alloc pinned staging");
+    CK(cudaHostGetDevicePointer((void **)&s->stage_dev, s->h_xfer, 0), "map pinned staging");
     CK(tg::xfer_prepare(s->prec), "load transfer kernels");
     s->h_err = reinterpret_cast<int *>(s->h_xfer + 9 * s->n);
     CK(cudaMemset(a.state0, 0, s->comps() * np * rs), "clear state");
@@ -2196,26 +2223,23 @@ int titan_gb300_get_masses(titan_gb300_sim *s, int64_t count, const int64_t *idx
         x.idx = s->d_idx;
     }
     // only the requested arrays come back: the kernel writes them into a
-    // page-locked caller buffer, else into the handle's staging buffer, and
+    // caller buffer that is page-locked as a whole, else into the handle's staging buffer, and
     // the error flag beside that
     double *outs[3] = {pos, vel, acc}, *dst[3] = {nullptr, nullptr, nullptr};
     bool direct[3] = {false, false, false};
-    double *const stage = (double *)host_on_device(s->h_xfer);
-    int *const err_dst = (int *)host_on_device(s->h_err);
     const bool any = pos || vel || acc;
     if (any) {
-        if (!stage || !err_dst) return s->fail(TITAN_GB300_ECUDA, "the staging buffer is not mapped");
         for (int q = 0; q < 3; q++) {
             if (!outs[q]) continue;
-            double *const h = (double *)host_on_device(outs[q]);
+            double *const h = (double *)host_on_device(outs[q], 3 * (size_t)count * 8);
             direct[q] = h && (reinterpret_cast<uintptr_t>(h) & 7) == 0;
-            dst[q] = direct[q] ? h : stage + 3 * q * count;
+            dst[q] = direct[q] ? h : s->stage_dev + 3 * q * count;
         }
         x.pos = dst[0];
         x.vel = dst[1];
         x.accout = dst[2];
         x.err = s->d_err;
-        x.err_out = err_dst;
+        x.err_out = reinterpret_cast<int *>(s->stage_dev + 9 * s->n);
         CK(tg::launch_gather(s->prec, x, s->stream), "gather");
     }
     CK(cudaStreamSynchronize(s->stream), "download");
