@@ -204,6 +204,15 @@ int titan_gb300_set_kernel(titan_gb300_sim *sim, int variant);
  * memory per CTA (bytes) -- of the resident-tile launch for form 5. */
 int titan_gb300_kernel_info(const titan_gb300_sim *sim, int64_t out[4]);
 
+/* After start(): how calls of step() run that all tiles take at once
+ * (set_kernel 0).  out[0] 1 when the scene has that form, else all are 0;
+ * out[1] tiles, a CTA each; out[2] threads per CTA; out[3] dynamic shared
+ * memory per CTA (bytes); out[4] 1 when the tiles' tables are in shared
+ * memory; out[5] 1 for the FP64 form with a lane per component; out[6] 1
+ * when single steps are one pass of the same kernel; out[7] the last step():
+ * 1 ran in that form, 2 as such a pass, 0 on other kernels. */
+int titan_gb300_grid_info(const titan_gb300_sim *sim, int64_t out[8]);
+
 /* Batched bodies (no reference counterpart: the reference runs one scene
  * per process, src/sim.cu:1503-1617).  With resident bins on, every body
  * (set_bodies) that fits one CTA -- no spring to another body, every free

@@ -68,6 +68,7 @@ _SIGS = {
     "titan_gb300_set_kernel": (ctypes.c_int, [_P, ctypes.c_int]),
     "titan_gb300_set_occupancy": (ctypes.c_int, [_P, ctypes.c_int]),
     "titan_gb300_kernel_info": (ctypes.c_int, [_P, _I64]),
+    "titan_gb300_grid_info": (ctypes.c_int, [_P, _I64]),
     "titan_gb300_set_resident": (ctypes.c_int, [_P, ctypes.c_int, ctypes.c_int, ctypes.c_int]),
     "titan_gb300_resident_info": (ctypes.c_int, [_P, _I64]),
     "titan_gb300_step": (ctypes.c_int, [_P, ctypes.c_int64]),
@@ -331,6 +332,15 @@ class Sim:
         names = {1: "per-tile", 3: "per-tile-async", 4: "warp-specialised", 5: "resident-tiles", 6: "pull"}
         return {"kernel": names.get(int(out[0]), "per-tile"), "ctas": int(out[1]), "threads": int(out[2]),
                 "smem_bytes": int(out[3])}
+
+    def grid_info(self) -> dict:
+        """How calls of step() run that all tiles take at once; last: the
+        last step() ran in that form (1), as a single pass of its kernel (2)
+        or on other kernels (0)."""
+        out = np.zeros(8, np.int64)
+        self._check(self._L.titan_gb300_grid_info(self._h, _ptr(out, ctypes.c_int64)), "grid_info")
+        keys = ("active", "tiles", "threads", "smem_bytes", "staged", "lanes", "single", "last")
+        return {k: int(v) for k, v in zip(keys, out)}
 
     def set_resident(self, mode: int = 1, bin_masses: int = 0, threads: int = 0):
         """Resident launches (all steps of a call in one kernel): mode -1

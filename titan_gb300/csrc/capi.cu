@@ -174,8 +174,9 @@ struct titan_gb300_sim {
     // for single steps
     bool use_grid = false;
     tg::GridResArgs gargs{};
-    int grid_shape = 0;
+    int grid_shape = 0, single_shape = -1;  // single steps as one pass of it, -1: by the per-step kernels
     size_t grid_smem = 0;
+    int grid_last = 0;  // the last step(): 1 resident grid, 2 its single pass, 0 other kernels
     // plan taken from another handle with the same topology (adopt_plan);
     // used by the first start() only
     bool plan_adopted = false;
@@ -532,6 +533,11 @@ constexpr int kPullDefaultTile = 224;
 constexpr bool kPullAuto = false;
 constexpr int kHeavyThreshold = 96;
 constexpr int64_t kGridMinSteps = 2;
+// Single steps of a scene planned for the resident grid run as one pass of
+// its kernel up to this many masses a tile (26^3: 5.9 us against 6.5 with
+// the warp-specialised kernel; 30^3, 89 masses a tile: 7.8 against 7.0), with
+// 256 threads a CTA (12^3: 4.0 us against 4.4 with 128).
+constexpr int kSingleMasses = 64, kSingleShape = 1;
 
 // Steps of one resident-grid launch: other handles' kernels get no SM that its
 // CTAs fill until it ends, so long calls are cut (100 steps of a 24^3 scene
@@ -1199,6 +1205,8 @@ int build_device(titan_gb300_sim *s) {
     }
     DEVCOPY(a.halo, P.halo, "upload halo");
     s->gargs = tg::GridResArgs{};
+    s->single_shape = -1;
+    s->grid_last = 0;
     s->use_grid = !tiles_run.empty() && grid_wanted(s) && !s->use_pull &&
                   choose_grid(s, tiles, s->grid_shape, s->gargs.stage, s->grid_smem);
     if (s->use_grid) {
@@ -1210,6 +1218,9 @@ int build_device(titan_gb300_sim *s) {
             if (!s->fixed.empty() && s->fixed[P.new2old[h]]) h = -1;
             else exported[h] = 1;
         }
+        if (s->prec != P_FP64 && s->gargs.stage && P.max_nm <= kSingleMasses &&
+            (int64_t)tiles.size() <= (int64_t)sms_dev * tg::grid_resident_ctas(kSingleShape))
+            s->single_shape = kSingleShape;
         if (s->use_rtiles) DEVCOPY(s->gargs.tiles, tiles, "upload tiles");
         else s->gargs.tiles = a.tiles;
         DEVCOPY(s->gargs.halo, halo, "upload halo");
@@ -1396,6 +1407,14 @@ bool ensure_device(titan_gb300_sim *s) { return cudaSetDevice(s->device) == cuda
 // per-step path decides, as without the resident grid.
 bool grid_runs(titan_gb300_sim *s, int64_t nsteps) {
     if (!s->use_grid || nsteps < kGridMinSteps) return false;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+}
+
+// Whether this call is a single step that runs as one pass of the resident
+// grid's kernel.
+bool single_runs(titan_gb300_sim *s, int64_t nsteps) {
+    if (!s->use_grid || s->single_shape < 0 || nsteps != 1) return false;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(s->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
 }
@@ -1610,6 +1629,21 @@ int titan_gb300_resident_info(const titan_gb300_sim *s, int64_t out[8]) {
     out[5] = s->res_threads;
     out[6] = s->res_ctas;
     out[7] = (int64_t)tg::resident_smem_bytes(s->prec, s->rargs.cap);
+    return TITAN_GB300_OK;
+}
+
+int titan_gb300_grid_info(const titan_gb300_sim *s, int64_t out[8]) {
+    if (!s || !out) return TITAN_GB300_EINVAL;
+    std::fill(out, out + 8, 0);
+    if (!s->started || !s->use_grid) return TITAN_GB300_OK;
+    out[0] = 1;
+    out[1] = s->gargs.ntiles;
+    out[2] = tg::grid_resident_threads(s->grid_shape);
+    out[3] = (int64_t)s->grid_smem;
+    out[4] = s->gargs.stage;
+    out[5] = tg::grid_resident_lanes(s->prec, s->grid_shape, s->gargs.max_nm);
+    out[6] = s->single_shape >= 0;
+    out[7] = s->grid_last;
     return TITAN_GB300_OK;
 }
 
@@ -1977,7 +2011,24 @@ int titan_gb300_step(titan_gb300_sim *s, int64_t nsteps) try {
     if (nsteps == 0) return TITAN_GB300_OK;
     if (!ensure_device(s)) return s->fail(TITAN_GB300_ECUDA, "cudaSetDevice failed");
     cudaError_t e = cudaSuccess;
+    s->grid_last = 0;
+    if (single_runs(s, nsteps)) {
+        const int P = s->passes();
+        s->gargs.T0 = s->T;
+        for (int q = 0; q < P; q++) {
+            CK(tg::launch_grid_single(s->prec, s->integrator, s->args, s->gargs, s->single_shape, s->grid_smem,
+                                      s->parity, q, q == P - 1, s->stream, !s->tables_written),
+               "launch step");
+            s->tables_written = false;
+            s->parity ^= 1;
+            s->gargs.T0 = s->gargs.T0 + s->hprm.launch_dt;
+        }
+        advance_clock(s, 1);
+        s->grid_last = 2;
+        return TITAN_GB300_OK;
+    }
     if (grid_runs(s, nsteps)) {
+        s->grid_last = 1;
         while (nsteps > 0 && s->use_grid) {
             const int64_t len = std::min(nsteps, kGridMaxSteps);
             s->gargs.T0 = s->T;
@@ -1994,6 +2045,7 @@ int titan_gb300_step(titan_gb300_sim *s, int64_t nsteps) try {
             if (r != cudaErrorCooperativeLaunchTooLarge) return s->cuda_fail(r, "launch resident grid");
             cudaGetLastError();
             s->use_grid = false;  // the device has less room than planned for: per-step kernels
+            s->grid_last = 0;
         }
         if (nsteps == 0) return TITAN_GB300_OK;
     }

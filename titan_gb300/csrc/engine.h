@@ -173,6 +173,8 @@ struct GridResArgs {
     double T0;                  // T of the launch's first step
     int32_t ntiles, max_nm;     // tiles, and the most masses of one
     int32_t stage;              // 1: slab, actuation and incidence records in shared memory
+    int32_t half;               // RK2: the half step that the launch's first pass is
+    int32_t single;             // a launch of one pass, by launch_grid_single
 };
 
 // Per-mass gather / scatter between caller order and tiled order.
@@ -282,8 +284,13 @@ size_t grid_resident_smem_bytes(int precision, const TileInfo &ti, int stage);
 int grid_resident_threads(int shape);
 int grid_resident_ctas(int shape);
 int grid_resident_exchange_bytes(int precision);
+bool grid_resident_lanes(int precision, int shape, int max_nm);  // a lane per component (epilogue_lanes.cuh)
 cudaError_t launch_grid_resident(int precision, int integ, const StepArgs &a, const GridResArgs &r, int shape,
                                  size_t smem, int parity, int64_t nsteps, int write_acc, cudaStream_t s);
+// One pass (RK2: half `half` of a step) as an ordinary launch, FP32 forms;
+// programmatic: it may start while the kernel before it on the stream drains.
+cudaError_t launch_grid_single(int precision, int integ, const StepArgs &a, const GridResArgs &r, int shape,
+                               size_t smem, int parity, int half, int write_acc, cudaStream_t s, bool programmatic);
 // loads the transfer kernels' code on the current device
 cudaError_t xfer_prepare(int precision);
 cudaError_t launch_gather(int precision, const XferArgs &a, cudaStream_t s);

@@ -30,11 +30,21 @@
 // (tile_phases.cuh, epilogue.cuh): the results are the same bits.  Waits are
 // bounded: a CTA that gives up raises *err, which the others poll.  The
 // launch is cooperative, so all CTAs run at once.
+//
+// A single step has no exchange, so its launch need not be cooperative: in
+// the FP32 forms it is one pass with programmatic stream serialisation, whose
+// CTAs stage their tables while the step before drains (launch_grid_single).
+// The tiles cut for this kernel are small for the warp-specialised one.  us
+// per step(1), FP32C, that kernel and this: 12^3 4.3 and 3.9, 16^3 5.3 and 4.2,
+// 20^3 5.8 and 4.7, 23^3 6.0 and 5.3, 26^3 6.5 and 5.9, 30^3 7.0 and 7.8 (there,
+// above 64 masses a tile, it is not used); with that kernel and its own larger
+// tiles 4.2, 4.2, 5.0, 5.5, 6.2 and 7.8.
 #include <cstdint>
 
 #include "engine.h"
 #include "epilogue.cuh"
 #include "epilogue_lanes.cuh"
+#include "grid_dep.cuh"
 #include "state.cuh"
 #include "step_math.cuh"
 #include "tile_phases.cuh"
@@ -92,6 +102,14 @@ __device__ __forceinline__ void st_chunk(void *p, const Chunk &c) {
                  : "memory");
 }
 
+// Data that the step before wrote.  In the FP32 forms around L1 and the
+// read-only path: a single step starts while that step still writes.
+template <int PREC, class T>
+__device__ __forceinline__ T load_fresh(const T *p) {
+    if constexpr (PREC == P_FP64) return __ldg(p);
+    else return __ldcg(p);
+}
+
 // The words of a state record that the exchange carries.
 template <int PREC>
 __device__ __forceinline__ void record_words(const St<PREC> &s, uint32_t *w) {
@@ -118,11 +136,10 @@ __device__ __forceinline__ void record_words(const St<PREC> &s, uint32_t *w) {
 
 template <int PREC, int INTEG, int STAGE, int SHAPE, bool LANES>
 __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
-    k_grid_resident(StepArgs a, GridResArgs r, int parity, int64_t nsteps, int write_acc) {
+    k_grid_resident(StepArgs a, GridResArgs r, int parity, int64_t passes, int write_acc) {
     using R = typename Real<PREC>::T;
     constexpr int kRec = PREC == P_FP32 ? 32 : 48;
     constexpr int kSlot = Slot<PREC>::kBytes;
-    constexpr int kPasses = INTEG == INTEG_RK2 ? 2 : 1;
     constexpr int kBatch = PREC == P_FP64 ? 1 : 3;  // slab entries a thread has in flight (measured best)
     constexpr int kChunks = PREC == P_FP32 ? 2 : 4;  // of one record in the exchange
     constexpr int kPoll = 4;                         // chunks a thread has in flight
@@ -143,13 +160,18 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
     const uint32_t inc_base = STAGE ? (uint32_t)ti.inc_off : 0u;
     const int64_t np = a.npad;
 
-    // the tile's state and tables
-    {
+    // the tile's state and tables; no step writes the tables, so a single step
+    // stages them before it waits for the one before
+    constexpr int kVec = kRec / 16;
+    auto load_tile = [&]() {
         const float4 *src = reinterpret_cast<const float4 *>(
             reinterpret_cast<const uint8_t *>(parity ? a.state1 : a.state0) + (int64_t)ti.mass_off * kRec);
-        for (int v = threadIdx.x; v < nm * (kRec / 16); v += blockDim.x)
-            reinterpret_cast<float4 *>(st)[v] = __ldg(src + v);
-    }
+        for (int v = threadIdx.x; v < nm * kVec; v += blockDim.x)
+            reinterpret_cast<float4 *>(st)[v] = load_fresh<PREC>(src + v);
+    };
+    const bool single = PREC != P_FP64 && r.single;
+    if constexpr (PREC == P_FP64) load_tile();
+    if (single) grid_dep_launch_dependents();
     if constexpr (STAGE) {
         for (int v = threadIdx.x; v < E * (kSlot / 16); v += blockDim.x)
             reinterpret_cast<float4 *>(smem + L.ent)[v] = __ldg(reinterpret_cast<const float4 *>(gent) + v);
@@ -202,11 +224,26 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
     // (written by CTA 0) when a CTA far from it starts
     double T = r.T0, Tbefore = T;
     const bool exported = i_own < nm && __ldg(r.exported + g_own) != 0;
+    // FP32 forms: the first halo masses of the first pass (the loads of their
+    // records then wait for nothing else)
+    constexpr int kAhead = PREC == P_FP64 ? 0 : 2;
+    int32_t hx[kAhead + 1];
+#pragma unroll
+    for (int k = 0; k < kAhead; k++) {
+        const int v = threadIdx.x + k * blockDim.x;
+        hx[k] = v < nh * kVec ? __ldg(a.halo + ti.halo_off + v / kVec) : 0;
+    }
+
+    if (single) grid_dep_wait();
+    if constexpr (PREC != P_FP64) load_tile();
     St<PREC> rk0;  // RK2: the step's starting state
+    if (PREC != P_FP64 && INTEG == INTEG_RK2 && r.half && i_own < nm)  // in the buffer this launch writes
+        rk0 = load_state<PREC, true>(parity ? a.state0 : a.state1, g_own);
     R acc0[3] = {0, 0, 0};  // VERLET: the acceleration of the step before
     if (INTEG == INTEG_VERLET && !(fl & MF_FIXED)) {
 #pragma unroll
-        for (int c = 0; c < 3; c++) acc0[c] = reinterpret_cast<const R *>(a.acc)[c * np + g_own];
+        for (int c = 0; c < 3; c++) acc0[c] = PREC == P_FP64 ? reinterpret_cast<const R *>(a.acc)[c * np + g_own]
+                                     : load_fresh<PREC>(reinterpret_cast<const R *>(a.acc) + c * np + g_own);
     }
     LaneMass lm{};
     double lx = 0.0, lv = 0.0;  // the lane's position and velocity
@@ -231,7 +268,6 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
         lm.md_ok = !alu_bad(bad) && alu_nonzero(y);
     }
     const bool lane_exported = LANES && lm.on && __ldg(r.exported + lm.g) != 0;
-    const int64_t passes = nsteps * kPasses;
     for (int64_t pass = 0; pass < passes; pass++) {
         // ---- A: the halo's records of the pass before ------------------------
         bool gave_up = false;
@@ -274,11 +310,15 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
             }
         } else {
             const uint8_t *in = reinterpret_cast<const uint8_t *>(parity ? a.state1 : a.state0);
-            for (int v = threadIdx.x; v < nh * (kRec / 16); v += blockDim.x)
-                reinterpret_cast<float4 *>(st + (int64_t)nm * kRec)[v] =
-                    __ldg(reinterpret_cast<const float4 *>(
-                              in + (int64_t)__ldg(a.halo + ti.halo_off + v / (kRec / 16)) * kRec) +
-                          v % (kRec / 16));
+            float4 *const to = reinterpret_cast<float4 *>(st + (int64_t)nm * kRec);
+            auto rec = [&](int32_t h, int v) {
+                return load_fresh<PREC>(reinterpret_cast<const float4 *>(in + (int64_t)h * kRec) + v % kVec);
+            };
+            int v = threadIdx.x;
+#pragma unroll
+            for (int k = 0; k < kAhead; k++, v += blockDim.x)
+                if (v < nh * kVec) to[v] = rec(hx[k], v);
+            for (; v < nh * kVec; v += blockDim.x) to[v] = rec(__ldg(a.halo + ti.halo_off + v / kVec), v);
         }
         if (__syncthreads_or(gave_up)) {
             if (threadIdx.x == 0) atomicOr(a.err, 1);
@@ -374,7 +414,7 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
                 for (uint32_t w = 0; w < nw; w++) gather_word_padded<PREC>(slots, word(w), F0, F1, F2);
             }
             St<PREC> s = load_state_smem<PREC>(st, i_own);
-            const int rk2_stage = INTEG == INTEG_RK2 ? (int)(pass & 1) : 0;
+            const int rk2_stage = INTEG == INTEG_RK2 ? (int)(pass & 1) ^ (PREC == P_FP64 ? 0 : r.half) : 0;
             if (INTEG == INTEG_RK2 && rk2_stage == 0) rk0 = s;
             integrate<PREC, INTEG>(a, ti, g_own, fl, m, F0, F1, F2, s, st, i_own, write_acc && pass == passes - 1, np,
                                    prm, rk2_stage, &rk0, INTEG == INTEG_VERLET ? acc0 : nullptr);
@@ -420,12 +460,9 @@ const void *rg_kernel(int integ, int stage, int shape) {
 // of at most kLaneWarps warps of masses (20^3 lattice, 53 masses: 12.5 us per
 // step against 12.9; 24^3, 91 masses: equal, with spills against none)
 const void *rg_kernel(int precision, int integ, int stage, int shape, int max_nm) {
-    if (precision == P_FP64) {
-        const int warps = kShapes[shape].threads / 32;
-        return max_nm <= kLaneMasses * (warps < kLaneWarps ? warps : kLaneWarps)
-                   ? rg_kernel<P_FP64, true>(integ, stage, shape)
-                   : rg_kernel<P_FP64, false>(integ, stage, shape);
-    }
+    if (precision == P_FP64)
+        return grid_resident_lanes(precision, shape, max_nm) ? rg_kernel<P_FP64, true>(integ, stage, shape)
+                                                             : rg_kernel<P_FP64, false>(integ, stage, shape);
     return precision == P_FP32 ? rg_kernel<P_FP32, false>(integ, stage, shape)
                                : rg_kernel<P_FP32C, false>(integ, stage, shape);
 }
@@ -439,14 +476,33 @@ int grid_resident_threads(int shape) { return kShapes[shape].threads; }
 int grid_resident_exchange_bytes(int precision) { return precision == P_FP32 ? 32 : 64; }
 
 int grid_resident_ctas(int shape) { return kShapes[shape].ctas; }
+bool grid_resident_lanes(int precision, int shape, int max_nm) {
+    const int warps = kShapes[shape].threads / 32;
+    return precision == P_FP64 && max_nm <= kLaneMasses * (warps < kLaneWarps ? warps : kLaneWarps);
+}
 
 cudaError_t launch_grid_resident(int precision, int integ, const StepArgs &a, const GridResArgs &r, int shape,
                                  size_t smem, int parity, int64_t nsteps, int write_acc, cudaStream_t s) {
     const void *f = rg_kernel(precision, integ, r.stage, shape, r.max_nm);
     const cudaError_t e = raise_smem_limit(f, smem);
     if (e != cudaSuccess) return e;
-    void *args[] = {const_cast<StepArgs *>(&a), const_cast<GridResArgs *>(&r), &parity, &nsteps, &write_acc};
+    int64_t passes = nsteps * (integ == INTEG_RK2 ? 2 : 1);
+    void *args[] = {const_cast<StepArgs *>(&a), const_cast<GridResArgs *>(&r), &parity, &passes, &write_acc};
     return cudaLaunchCooperativeKernel(f, dim3(r.ntiles), dim3(kShapes[shape].threads), args, smem, s);
+}
+
+cudaError_t launch_grid_single(int precision, int integ, const StepArgs &a, const GridResArgs &r, int shape,
+                               size_t smem, int parity, int half, int write_acc, cudaStream_t s, bool programmatic) {
+    if (precision == P_FP64) return cudaErrorInvalidValue;
+    const void *f = rg_kernel(precision, integ, r.stage, shape, r.max_nm);
+    const cudaError_t e = raise_smem_limit(f, smem);
+    if (e != cudaSuccess) return e;
+    GridResArgs one = r;
+    one.half = half;
+    one.single = 1;
+    int64_t passes = 1;
+    void *args[] = {const_cast<StepArgs *>(&a), &one, &parity, &passes, &write_acc};
+    return launch_programmatic(f, dim3(r.ntiles), dim3(kShapes[shape].threads), args, smem, s, programmatic);
 }
 
 }  // namespace tg

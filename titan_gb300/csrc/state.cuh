@@ -19,25 +19,28 @@ struct St<P_FP64> {
     double x[3], v[3], xl[3], vl[3];
 };
 
-template <int PREC>
+// FRESH: around L1, for records that a kernel still running may have written
+// since this SM last read them.
+template <int PREC, bool FRESH = false>
 __device__ __forceinline__ St<PREC> load_state(const void *buf, int64_t g) {
     St<PREC> s;
+    auto ld = [](const auto *p) { return FRESH ? __ldcg(p) : __ldg(p); };
     if constexpr (PREC == P_FP64) {
         const double2 *p = reinterpret_cast<const double2 *>(buf) + 3 * g;
-        double2 a0 = __ldg(p), a1 = __ldg(p + 1), a2 = __ldg(p + 2);
+        double2 a0 = ld(p), a1 = ld(p + 1), a2 = ld(p + 2);
         s.x[0] = a0.x; s.x[1] = a0.y; s.x[2] = a1.x;
         s.v[0] = a1.y; s.v[1] = a2.x; s.v[2] = a2.y;
     } else if constexpr (PREC == P_FP32C) {
         const float4 *p = reinterpret_cast<const float4 *>(buf) + 3 * g;
-        float4 a0 = __ldg(p), a1 = __ldg(p + 1), a2 = __ldg(p + 2);
+        float4 a0 = ld(p), a1 = ld(p + 1), a2 = ld(p + 2);
         s.x[0] = a0.x; s.x[1] = a0.y; s.x[2] = a0.z;
         s.v[0] = a0.w; s.v[1] = a1.x; s.v[2] = a1.y;
         s.xl[0] = a1.z; s.xl[1] = a1.w; s.xl[2] = a2.x;
         s.vl[0] = a2.y; s.vl[1] = a2.z; s.vl[2] = a2.w;
     } else {
         const float4 *p = reinterpret_cast<const float4 *>(buf) + 2 * g;
-        float4 a0 = __ldg(p);
-        float2 a1 = __ldg(reinterpret_cast<const float2 *>(p + 1));
+        float4 a0 = ld(p);
+        float2 a1 = ld(reinterpret_cast<const float2 *>(p + 1));
         s.x[0] = a0.x; s.x[1] = a0.y; s.x[2] = a0.z;
         s.v[0] = a0.w; s.v[1] = a1.x; s.v[2] = a1.y;
         s.xl[0] = s.xl[1] = s.xl[2] = 0.f;  // the epilogue adds the (zero) low parts
