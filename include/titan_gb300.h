@@ -205,12 +205,13 @@ int titan_gb300_set_kernel(titan_gb300_sim *sim, int variant);
 int titan_gb300_kernel_info(const titan_gb300_sim *sim, int64_t out[4]);
 
 /* After start(): how calls of step() run that all tiles take at once
- * (set_kernel 0).  out[0] 1 when the scene has that form, else all are 0;
+ * (set_kernel 0).  out[0] 1 when the scene has that form, else out[0..6] are 0;
  * out[1] tiles, a CTA each; out[2] threads per CTA; out[3] dynamic shared
  * memory per CTA (bytes); out[4] 1 when the tiles' tables are in shared
  * memory; out[5] 1 for the FP64 form with a lane per component; out[6] 1
  * when single steps are one pass of the same kernel; out[7] the last step():
- * 1 ran in that form, 2 as such a pass, 0 on other kernels. */
+ * 1 ran in that form, 2 as such a pass, 3 a call of a few steps on a scene
+ * of many bodies that longer calls keep resident, 0 other kernels. */
 int titan_gb300_grid_info(const titan_gb300_sim *sim, int64_t out[8]);
 
 /* Batched bodies (no reference counterpart: the reference runs one scene
@@ -257,7 +258,10 @@ int titan_gb300_step(titan_gb300_sim *sim, int64_t nsteps);
  * kernels directly): builds and caches the CUDA graphs that step(nsteps)
  * would replay from the current step parity, without launching anything, so
  * that a later step(nsteps) spends no host time on graph capture.  Graphs
- * are dropped when the scene is rebuilt (integrator switch, topology change). */
+ * are dropped when the scene is rebuilt (integrator switch, topology change).
+ * On scenes of many bodies that longer calls keep resident it makes the tables
+ * for calls of nsteps, if these are few, which step() makes at the 65th such
+ * call (device memory as for the bodies' spring records once more). */
 int titan_gb300_prepare_steps(titan_gb300_sim *sim, int64_t nsteps);
 
 /* Wait for queued work; replaces the cudaDeviceSynchronize at src/sim.cu:1570.

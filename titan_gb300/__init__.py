@@ -335,8 +335,9 @@ class Sim:
 
     def grid_info(self) -> dict:
         """How calls of step() run that all tiles take at once; last: the
-        last step() ran in that form (1), as a single pass of its kernel (2)
-        or on other kernels (0)."""
+        last step() ran in that form (1), as a single pass of its kernel (2),
+        as a call of a few steps of a scene of many bodies (3) or on other
+        kernels (0)."""
         out = np.zeros(8, np.int64)
         self._check(self._L.titan_gb300_grid_info(self._h, _ptr(out, ctypes.c_int64)), "grid_info")
         keys = ("active", "tiles", "threads", "smem_bytes", "staged", "lanes", "single", "last")

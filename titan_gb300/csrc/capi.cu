@@ -170,13 +170,24 @@ struct titan_gb300_sim {
         size_t smem = 0;
     };
     std::vector<RtGroup> rt_groups;
+    // calls of a few steps on scenes with whole bodies above the per-step
+    // tile size (short_limit): those bodies in pieces of that size.  The
+    // tables are the plan's and behind them the pieces'.
+    struct ShortForm {
+        bool tried = false, ready = false;
+        int64_t calls = 0;  // such calls before the tables were made
+        tg::StepArgs args{};
+        tg::RepeatArgs pieces{};
+        int ctas = 0;
+    } short_form;
+    double *d_t0 = nullptr;  // the first step's T, where per-step kernels advance the record beside them
     // all tiles at once (resident_grid.cu); the per-step kernels stay ready
     // for single steps
     bool use_grid = false;
     tg::GridResArgs gargs{};
     int grid_shape = 0, single_shape = -1;  // single steps as one pass of it, -1: by the per-step kernels
     size_t grid_smem = 0;
-    int grid_last = 0;  // the last step(): 1 resident grid, 2 its single pass, 0 other kernels
+    int grid_last = 0;  // the last step(): 1 resident grid, 2 its single pass, 3 short_form, 0 other kernels
     // plan taken from another handle with the same topology (adopt_plan);
     // used by the first start() only
     bool plan_adopted = false;
@@ -218,6 +229,7 @@ struct titan_gb300_sim {
         d_partials = d_dout = nullptr;
         for (int q = 0; q < SP_COUNT; q++) d_sp[q] = nullptr, sp_current[q] = false;
         d_espring = nullptr;
+        short_form = ShortForm{};
     }
     ~titan_gb300_sim() {
         if (stream) cudaStreamSynchronize(stream);
@@ -484,6 +496,17 @@ int upload_records(titan_gb300_sim *s, const std::vector<int64_t> &spring, const
     return TITAN_GB300_OK;
 }
 
+// The records of the tables for calls of a few steps, from the plan's.
+int refresh_short(titan_gb300_sim *s) {
+    const auto &f = s->short_form;
+    const size_t bytes = s->plan.ent_ends.size() * (size_t)tg::entry_record_bytes(s->prec);
+    CK(cudaMemcpyAsync(const_cast<void *>(f.args.ent), s->args.ent, bytes, cudaMemcpyDeviceToDevice, s->stream), "copy records");
+    CK(cudaMemcpyAsync(const_cast<void *>(f.args.act), s->args.act, bytes, cudaMemcpyDeviceToDevice, s->stream), "copy records");
+    CK(tg::launch_repeat_entries(s->prec, f.pieces, s->stream), "repeat records");
+    s->tables_written = true;
+    return TITAN_GB300_OK;
+}
+
 // Slab entry records and actuation parameters from the host spring arrays,
 // and the resident bins' records.
 int upload_entries(titan_gb300_sim *s) {
@@ -506,6 +529,8 @@ int upload_entries(titan_gb300_sim *s) {
                       cudaMemcpyHostToDevice),
            "upload pull columns");
     }
+    if (s->short_form.ready)
+        if (int rs = refresh_short(s)) return rs;
     if (s->use_res)
         rc = upload_records(s, s->rplan.rec_spring, s->rplan.words, const_cast<void *>(s->rargs.rec),
                             const_cast<void *>(s->rargs.act));
@@ -699,10 +724,13 @@ tg::PlanInput plan_input(titan_gb300_sim *s, int tile_masses, bool grid = false)
             // many bodies: whole ones of up to 512 masses run resident
             // (Euler), a step of 608 bodies of 6^3 masses in 8.9 us against
             // 16.5 as two tiles each, of 8^3 in 24.8 against 30.7; of 9^3 in
-            // 42.6 either way
+            // 42.6 either way.  Calls of a few steps take those bodies in
+            // tiles of the size above (short_limit), over the same masses
             if (grid_wanted(s) && s->integrator == tg::INTEG_EULER &&
-                (int64_t)s->body_ptr.size() > 2 * (int64_t)sms)
+                (int64_t)s->body_ptr.size() > 2 * (int64_t)sms) {
                 in.whole_cap = 512;
+                in.cut_above = kWsDefaultTile;
+            }
         } else {
             in.tile_cap = 256;
         }
@@ -804,6 +832,18 @@ void ws_stage_layout(int prec, const std::vector<tg::TileInfo> &tiles, tg::WsLay
                          (2 * tg::kWsMaxStages + 2) * 8 + 32;
     const int64_t room = 227 * 1024 - tail;
     W.nstages = (int32_t)std::min<int64_t>(tg::kWsMaxStages, room / std::max<int64_t>(1, W.stage));
+}
+
+// The rest of the layout, behind W.nstages >= 2 stages.
+void ws_tail_layout(int prec, tg::WsLayout &W) {
+    auto al = [](int64_t x, int64_t q) { return (x + q - 1) / q * q; };
+    const int64_t rs = prec == P_FP64 ? 8 : 4;
+    W.idx = W.nstages * W.stage;
+    W.heavy = W.idx + 2 * W.idx_words * 4;
+    W.tinfo = (int32_t)al(W.heavy + 2 * 3 * (int64_t)W.heavy_cap * rs, 16);
+    W.params = W.tinfo + W.nstages * (int32_t)sizeof(tg::TileInfo);
+    W.mbar = (int32_t)al(W.params + (int64_t)sizeof(tg::DevParams), 16);
+    W.total = W.mbar + (2 * W.nstages + 2) * 8 + 32;
 }
 
 // Shared-memory layout of the pull kernel for these tiles (sized by their
@@ -953,8 +993,114 @@ int refresh_entries(titan_gb300_sim *s, unsigned given) {
         x.par[q] = s->d_sp[q];
     }
     CK(tg::launch_entries(s->prec, x, s->stream), "refresh entries");
+    if (s->short_form.ready)
+        if (int rc = refresh_short(s)) return rc;
     s->tables_written = true;
     return TITAN_GB300_OK;
+}
+
+// Calls of at most this many steps run the warp-specialised kernel on tiles
+// of its own size (build_short) although whole bodies are resident: a launch
+// of resident bodies costs 12 to 30 us more than its steps and is bound by its
+// largest bodies (a CTA of 512 masses fills an SM).  Measured, FP32C, us per
+// call with resident bodies and with this: 608 bodies of 6^3 masses, 1 step 18
+// and 16, 2 steps 32 and 41; of 8^3, 1 step 56 and 31, 4 steps 130 and 129;
+// beside bodies too large to be resident, 320 of 6^3 to 9^3, 1 step 31 and 17,
+// 6 steps 114 and 107; 600 of 3^3 to 9^3, 1 step 31 and 21, 6 steps 140 and
+// 131, 12 steps 257 and 252; 1024 of 3^3 to 12^3, 1 step 94 and 71, 4 steps
+// 296 and 292, 8 steps 552 and 572.
+int short_limit(const titan_gb300_sim *s) {
+    if (!s->use_rtiles || s->use_grid || s->prec == P_FP64 || !grid_wanted(s) || s->tile_masses > 0) return 0;
+    int largest = 0;
+    for (const tg::TileInfo &ti : s->rtiles) largest = std::max(largest, (int)ti.nm);
+    if (largest <= kWsDefaultTile) return 0;
+    if (s->args.ntiles > 0) return s->n <= 1500 * (int64_t)sm_count(s) ? 12 : 6;
+    return largest <= 256 ? 1 : 4;
+}
+
+// The tables of those tiles, made at the 65th such call (or by
+// prepare_steps): they take 5 to 75 ms (320 bodies of 3^3 to 9^3 11 ms, 608 of
+// 8^3 61), a quarter to a half of start(), which a scene that takes a few
+// short calls only would not get back.  Without room for them the resident
+// bodies serve these calls too.
+constexpr int64_t kShortCalls = 64;
+int build_short(titan_gb300_sim *s) {
+    auto &f = s->short_form;
+    if (f.tried) return TITAN_GB300_OK;
+    f.tried = true;
+    const tg::Plan &P = s->plan;
+    std::vector<tg::TileInfo> tiles;
+    std::vector<int64_t> whole;
+    for (const tg::TileInfo &ti : tile_infos(P)) {
+        const bool cut = ti.nh == 0 && ti.nm > kWsDefaultTile;
+        if (cut && ti.nheavy > 0) return TITAN_GB300_OK;
+        if (cut) whole.push_back((int64_t)(std::upper_bound(P.tile_mass_off.begin(), P.tile_mass_off.end(), ti.mass_off) -
+                                           P.tile_mass_off.begin()) - 1);
+        else tiles.push_back(ti);
+    }
+    const std::vector<tg::CutTile> cuts = tg::cut_tiles(P, whole, tg::state_record_bytes(s->prec));
+    // where the pieces' tables start behind the plan's
+    const int64_t E = (int64_t)P.ent_ends.size();
+    std::vector<int32_t> halo(P.halo), src;
+    std::vector<uint32_t> warp_inc(P.warp_inc_off), ends;
+    std::vector<uint16_t> inc(P.inc);
+    for (const tg::CutTile &c : cuts) {
+        tg::TileInfo ti{};
+        ti.mass_off = (int32_t)c.lo;
+        ti.nm = (int32_t)(c.hi - c.lo);
+        ti.halo_off = (int32_t)halo.size();
+        ti.nh = c.nh;
+        ti.ent_off = (int32_t)(E + (int64_t)src.size());
+        ti.ne = (int32_t)c.entry.size();
+        ti.nact = c.nact;
+        ti.warp_off = (int32_t)warp_inc.size();
+        ti.body = c.body;
+        ti.inc_off = (int32_t)inc.size();
+        ti.inc_words = (int32_t)c.inc.size();
+        tiles.push_back(ti);
+        for (const uint32_t w : c.warp_inc) warp_inc.push_back((uint32_t)inc.size() + w);
+        halo.insert(halo.end(), c.halo.begin(), c.halo.end());
+        src.insert(src.end(), c.entry.begin(), c.entry.end());
+        ends.insert(ends.end(), c.ends.begin(), c.ends.end());
+        inc.insert(inc.end(), c.inc.begin(), c.inc.end());
+    }
+    if (E + src.size() > (size_t)INT32_MAX || halo.size() > (size_t)INT32_MAX || inc.size() > (size_t)INT32_MAX)
+        return TITAN_GB300_OK;
+    f.args = s->args;
+    tg::StepArgs &a = f.args;
+    ws_stage_layout(s->prec, tiles, a.ws);
+    if (a.ws.nstages < 2) return TITAN_GB300_OK;
+    ws_tail_layout(s->prec, a.ws);
+    cudaError_t e = tg::step_ws_prepare(s->prec, tg::INTEG_EULER, (size_t)a.ws.total);
+    const size_t rec = (E + src.size()) * tg::entry_record_bytes(s->prec);
+    int32_t *d_src = nullptr;
+    uint32_t *d_ends = nullptr;
+    if (e != cudaSuccess || !(a.tiles = dev_copy(s, tiles, e)) || !(a.halo = dev_copy(s, halo, e)) ||
+        !(a.warp_inc_off = dev_copy(s, warp_inc, e)) || !(a.inc = dev_copy(s, inc, e)) ||
+        !(d_src = dev_copy(s, src, e)) || !(d_ends = dev_copy(s, ends, e)) || !(a.ent = s->mem.get(rec, e)) ||
+        !(a.act = s->mem.get(rec, e))) {
+        cudaGetLastError();
+        return e == cudaErrorMemoryAllocation ? TITAN_GB300_OK : s->cuda_fail(e, "tables for calls of a few steps");
+    }
+    f.pieces = tg::RepeatArgs{d_src, d_ends, const_cast<void *>(a.ent), const_cast<void *>(a.act), E, (int64_t)src.size()};
+    a.ntiles = (int32_t)tiles.size();
+    f.ctas = (int)std::min<int64_t>((int64_t)tiles.size(), sm_count(s));
+    f.ready = true;
+    return refresh_short(s);
+}
+
+// Whether a call of nsteps runs in those tiles; makes their tables when there
+// have been enough such calls, or at once (now).
+bool short_runs(titan_gb300_sim *s, int64_t nsteps, bool now, int &rc) {
+    rc = TITAN_GB300_OK;
+    if (nsteps > short_limit(s)) return false;
+    if (!s->short_form.tried) {
+        if (!now && ++s->short_form.calls <= kShortCalls) return false;
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return false;
+        rc = build_short(s);
+    }
+    return rc == TITAN_GB300_OK && s->short_form.ready;
 }
 
 // Builds the plan and all device buffers; positions/velocities come from the
@@ -1129,14 +1275,8 @@ int build_device(titan_gb300_sim *s) {
             return s->fail(TITAN_GB300_ELIMIT, "two tiles do not fit in shared memory for the warp-specialised kernel");
     }
     if (want_ws && a.ws.nstages >= 2) {
-        auto al = [](int64_t x, int64_t q) { return (x + q - 1) / q * q; };
         tg::WsLayout &W = a.ws;
-        W.idx = W.nstages * W.stage;
-        W.heavy = W.idx + 2 * W.idx_words * 4;
-        W.tinfo = (int32_t)al(W.heavy + 2 * 3 * (int64_t)W.heavy_cap * (int64_t)rs, 16);
-        W.params = W.tinfo + W.nstages * (int32_t)sizeof(tg::TileInfo);
-        W.mbar = (int32_t)al(W.params + (int64_t)sizeof(tg::DevParams), 16);
-        W.total = W.mbar + (2 * W.nstages + 2) * 8 + 32;
+        ws_tail_layout(s->prec, W);
         s->ws_warps = s->threads_req > 0 ? s->threads_req / 32 : tg::kWsMaxConsumerWarps;
         s->ws_warps = std::max(2, std::min(tg::kWsMaxConsumerWarps, s->ws_warps)) & ~1;
         CK(tg::step_ws_prepare(s->prec, s->integrator, (size_t)W.total), "set shared memory");
@@ -1259,11 +1399,9 @@ int build_device(titan_gb300_sim *s) {
     if (!(a.acc = s->mem.get(3 * np * rs, e))) return s->cuda_fail(e, "alloc acc");
     if (!(a.tbuf = (double *)s->mem.get(2 * sizeof(double), e))) return s->cuda_fail(e, "alloc time");
     if (s->use_rtiles) {
-        const double *t0 = (const double *)s->mem.get(sizeof(double), e);
-        if (!t0) return s->cuda_fail(e, "alloc time");
+        if (!(s->d_t0 = (double *)s->mem.get(sizeof(double), e))) return s->cuda_fail(e, "alloc time");
         if (!s->ev_fork) CK(cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming), "create event");
         for (size_t q = 0; q < s->rt_groups.size(); q++) {
-            s->rt_groups[q].args.t0 = t0;
             if (!s->side_stream[q])
                 CK(cudaStreamCreateWithFlags(&s->side_stream[q], cudaStreamNonBlocking), "create stream");
             if (!s->ev_join[q]) CK(cudaEventCreateWithFlags(&s->ev_join[q], cudaEventDisableTiming), "create event");
@@ -1635,7 +1773,9 @@ int titan_gb300_resident_info(const titan_gb300_sim *s, int64_t out[8]) {
 int titan_gb300_grid_info(const titan_gb300_sim *s, int64_t out[8]) {
     if (!s || !out) return TITAN_GB300_EINVAL;
     std::fill(out, out + 8, 0);
-    if (!s->started || !s->use_grid) return TITAN_GB300_OK;
+    if (!s->started) return TITAN_GB300_OK;
+    out[7] = s->grid_last;
+    if (!s->use_grid) return TITAN_GB300_OK;
     out[0] = 1;
     out[1] = s->gargs.ntiles;
     out[2] = tg::grid_resident_threads(s->grid_shape);
@@ -1643,7 +1783,6 @@ int titan_gb300_grid_info(const titan_gb300_sim *s, int64_t out[8]) {
     out[4] = s->gargs.stage;
     out[5] = tg::grid_resident_lanes(s->prec, s->grid_shape, s->gargs.max_nm);
     out[6] = s->single_shape >= 0;
-    out[7] = s->grid_last;
     return TITAN_GB300_OK;
 }
 
@@ -2027,6 +2166,20 @@ int titan_gb300_step(titan_gb300_sim *s, int64_t nsteps) try {
         s->grid_last = 2;
         return TITAN_GB300_OK;
     }
+    int rc_short = TITAN_GB300_OK;
+    if (short_runs(s, nsteps, false, rc_short)) {
+        for (int64_t i = 0; i < nsteps; i++) {
+            CK(tg::launch_step_ws(s->prec, s->integrator, s->short_form.args, s->short_form.ctas,
+                                  tg::kWsMaxConsumerWarps, s->parity, i == nsteps - 1, s->stream, !s->tables_written),
+               "launch step");
+            s->tables_written = false;
+            s->parity ^= 1;
+        }
+        advance_clock(s, nsteps);
+        s->grid_last = 3;
+        return TITAN_GB300_OK;
+    }
+    if (rc_short) return rc_short;
     if (grid_runs(s, nsteps)) {
         s->grid_last = 1;
         while (nsteps > 0 && s->use_grid) {
@@ -2055,10 +2208,16 @@ int titan_gb300_step(titan_gb300_sim *s, int64_t nsteps) try {
            "launch resident bins");
     const bool alone = s->args.ntiles == 0;
     if (s->use_rtiles) {
-        // the first step's time, copied before per-step kernels advance the record
-        CK(cudaMemcpyAsync(const_cast<double *>(s->rt_groups[0].args.t0), s->args.tbuf + s->parity, sizeof(double),
-                           cudaMemcpyDeviceToDevice, s->stream),
-           "launch resident tiles");
+        // the first step's time: of the record's two places a step reads one and
+        // writes the other, so a copy is needed only where per-step kernels
+        // take more than one step beside the launch
+        const double *t0 = s->args.tbuf + s->parity;
+        if (!alone && nsteps > 1) {
+            t0 = s->d_t0;
+            CK(cudaMemcpyAsync(s->d_t0, s->args.tbuf + s->parity, sizeof(double), cudaMemcpyDeviceToDevice, s->stream),
+               "launch resident tiles");
+        }
+        const bool own_time = alone && (nsteps & 1);
         // beside the per-step kernels and each other: disjoint masses (the
         // first group of a scene without per-step tiles needs no side stream)
         const size_t first = alone ? 1 : 0;
@@ -2067,14 +2226,17 @@ int titan_gb300_step(titan_gb300_sim *s, int64_t nsteps) try {
             const auto &g = s->rt_groups[q];
             cudaStream_t st = q < first ? s->stream : s->side_stream[q];
             if (q >= first) CK(cudaStreamWaitEvent(st, s->ev_fork, 0), "launch resident tiles");
-            CK(tg::launch_tile_resident(s->prec, s->args, g.args, g.mpt, g.threads, g.smem, s->parity, nsteps, 1, st),
+            tg::TileResArgs r = g.args;
+            r.t0 = t0;
+            if (own_time && q == 0) r.time = s->args.tbuf + (s->parity ^ 1);
+            CK(tg::launch_tile_resident(s->prec, s->args, r, g.mpt, g.threads, g.smem, s->parity, nsteps, 1, st),
                "launch resident tiles");
             if (q >= first) CK(cudaEventRecord(s->ev_join[q], st), "launch resident tiles");
         }
         if (alone) {
             for (size_t q = first; q < s->rt_groups.size(); q++)
                 CK(cudaStreamWaitEvent(s->stream, s->ev_join[q], 0), "join resident tiles");
-            CK(tg::launch_advance_time(s->args, s->parity, nsteps, s->stream), "advance time");
+            if (!own_time) CK(tg::launch_advance_time(s->args, s->parity, nsteps, s->stream), "advance time");
         }
     }
     if (s->args.ntiles == 0) {
@@ -2118,8 +2280,9 @@ int titan_gb300_prepare_steps(titan_gb300_sim *s, int64_t nsteps) try {
     if (s->serving) return s->fail(TITAN_GB300_ESTATE, "the scene is being stepped by a request server");
     if (!s->started) return s->fail(TITAN_GB300_ESTATE, "The simulation has not started.");
     if (nsteps < 0) return s->fail(TITAN_GB300_EINVAL, "negative step count");
-    if (s->args.ntiles == 0 || nsteps <= 1 || grid_runs(s, nsteps)) return TITAN_GB300_OK;
     if (!ensure_device(s)) return s->fail(TITAN_GB300_ECUDA, "cudaSetDevice failed");
+    if (int rc = TITAN_GB300_OK; nsteps > 0 && (short_runs(s, nsteps, true, rc) || rc)) return rc;
+    if (s->args.ntiles == 0 || nsteps <= 1 || grid_runs(s, nsteps)) return TITAN_GB300_OK;
     // the same chunk sequence step(nsteps) replays, from the current parity
     cudaError_t e = cudaSuccess;
     const int P = s->passes();

@@ -156,7 +156,8 @@ struct ResArgs {
 // of a launch, with the per-step kernels' two phases in shared memory.
 struct TileResArgs {
     const TileInfo *tiles;  // the resident tiles
-    const double *t0;       // T of the launch's first step (a copy taken before per-step kernels run beside it)
+    const double *t0;       // T of the launch's first step (nothing that runs beside the launch writes there)
+    double *time;           // CTA 0 writes T after the launch there, if given
     int32_t ntiles;
     int32_t stage;          // 1: slab, actuation and incidence records staged in shared memory once per launch
 };
@@ -200,6 +201,15 @@ struct EntryArgs {
     void *rec, *act;
     int64_t count;
     const double *par[6];
+};
+
+// Slab records that repeat other entries' values with ends of their own:
+// record first + e is that of entry src[e] with the ends in ends[e].
+struct RepeatArgs {
+    const int32_t *src;
+    const uint32_t *ends;
+    void *rec, *act;
+    int64_t first, count;
 };
 
 struct DiagArgs {
@@ -299,6 +309,7 @@ cudaError_t launch_export_f32(int precision, const XferArgs &a, float *out, cuda
 cudaError_t launch_scatter(int precision, const XferArgs &a, cudaStream_t s);
 cudaError_t launch_diag(int precision, const DiagArgs &a, cudaStream_t s);
 cudaError_t launch_entries(int precision, const EntryArgs &a, cudaStream_t s);
+cudaError_t launch_repeat_entries(int precision, const RepeatArgs &a, cudaStream_t s);
 // a.count masses' raw records (rec) and accelerations (acc, component-major)
 // to caller order, or from it into both state buffers
 cudaError_t launch_carry(int precision, const XferArgs &a, bool out, void *rec, void *acc, cudaStream_t s);

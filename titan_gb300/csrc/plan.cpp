@@ -2,6 +2,7 @@
 #include "plan.h"
 
 #include <algorithm>
+#include <array>
 #include <system_error>
 #include <thread>
 #include <atomic>
@@ -523,6 +524,33 @@ void layout_leaf(const PlanInput &in, const Plan &P, const std::vector<int32_t> 
     }
 }
 
+// bank_order on a slab's actuated part and on the rest, which continues the
+// actuated part's last group.  left, right: the slots of an entry's ends.
+template <class Left, class Right>
+void bank_order_slab(std::vector<int64_t> &act, std::vector<int64_t> &rest, int slot_bytes, Left left, Right right) {
+    uint32_t lead_ls[8], lead_rs[8];
+    int lead = 0;
+    for (auto *v : {&act, &rest}) {
+        std::vector<uint32_t> ls(v->size()), rs(v->size());
+        for (size_t q = 0; q < v->size(); q++) {
+            ls[q] = left((*v)[q]);
+            rs[q] = right((*v)[q]);
+        }
+        bank_order(*v, ls, rs, slot_bytes, lead_ls, lead_rs, lead);
+        // the open group after this part: its last (lead + size) % 8
+        // entries of the carried ones followed by this part's
+        std::vector<uint32_t> cl(lead_ls, lead_ls + lead), cr(lead_rs, lead_rs + lead);
+        for (int64_t e : *v) {
+            cl.push_back(left(e));
+            cr.push_back(right(e));
+        }
+        const int tail = (int)(cl.size() % 8);
+        std::copy(cl.end() - tail, cl.end(), lead_ls);
+        std::copy(cr.end() - tail, cr.end(), lead_rs);
+        lead = tail;
+    }
+}
+
 // Final slab order of tile t (bank_order on each part, then
 // gather_permute), its entry words, and the incidence codes of its masses
 // (ELL block and heavy lists), written into the tile's own ranges of P's
@@ -541,30 +569,8 @@ void order_tile(const PlanInput &in, Plan &P, int64_t t, const std::vector<int32
     };
     std::vector<int64_t> ents_act(P.ent_spring.begin() + e0, P.ent_spring.begin() + e0 + na);
     std::vector<int64_t> ents(P.ent_spring.begin() + e0 + na, P.ent_spring.begin() + e1);
-    {
-        // the non-actuated part continues the actuated part's last group
-        uint32_t lead_ls[8], lead_rs[8];
-        int lead = 0;
-        for (auto *v : {&ents_act, &ents}) {
-            std::vector<uint32_t> ls(v->size()), rs(v->size());
-            for (size_t q = 0; q < v->size(); q++) {
-                ls[q] = slot(L[(*v)[q]]);
-                rs[q] = slot(R[(*v)[q]]);
-            }
-            bank_order(*v, ls, rs, in.slot_bytes, lead_ls, lead_rs, lead);
-            // the open group after this part: its last (lead + size) % 8
-            // entries of the carried ones followed by this part's
-            std::vector<uint32_t> cl(lead_ls, lead_ls + lead), cr(lead_rs, lead_rs + lead);
-            for (int64_t sp : *v) {
-                cl.push_back(slot(L[sp]));
-                cr.push_back(slot(R[sp]));
-            }
-            const int tail = (int)(cl.size() % 8);
-            std::copy(cl.end() - tail, cl.end(), lead_ls);
-            std::copy(cr.end() - tail, cr.end(), lead_rs);
-            lead = tail;
-        }
-    }
+    bank_order_slab(ents_act, ents, in.slot_bytes, [&](int64_t sp) { return slot(L[sp]); },
+                    [&](int64_t sp) { return slot(R[sp]); });
     gather_permute(ents_act, ents, lo, hi, ip, isp, in.heavy_threshold, W);
     W.begin(e1 - e0);
     int64_t e = e0;
@@ -635,7 +641,7 @@ static std::string build_plan_tables(const PlanInput &in, Plan &P) {
     std::vector<int64_t> leaf_end;  // new-index end of each leaf, in order
     // bodies on several threads (each writes only its own ranges); a lone
     // body cuts its top levels on several threads instead
-    std::vector<std::vector<int64_t>> body_leaves((size_t)P.nbodies);
+    std::vector<std::vector<int64_t>> body_leaves((size_t)P.nbodies), body_cuts((size_t)P.nbodies);
     parallel_items<NoScratch>(P.nbodies, 16, [&](NoScratch &, int64_t b) {
         int64_t b0 = bptr[b], b1 = bptr[b + 1];
         double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -662,11 +668,18 @@ static std::string build_plan_tables(const PlanInput &in, Plan &P) {
             }
             code[i] = spread21(q[0]) | (spread21(q[1]) << 1) | (spread21(q[2]) << 2);
         }
-        const int cap_b = (b1 - b0) <= (int64_t)in.whole_cap ? (int)(b1 - b0) : in.tile_cap;
+        const bool whole = (b1 - b0) <= (int64_t)in.whole_cap;
+        const bool cut = whole && in.cut_above > 0 && (b1 - b0) > (int64_t)in.cut_above;
+        const int cap_b = whole && !cut ? (int)(b1 - b0) : in.tile_cap;
         int depth = 0;  // a lone body: about one cut's half per thread
         while (P.nbodies == 1 && (2 << depth) <= planner_threads() && depth < 6) depth++;
         bisect(P.new2old.data() + b0, b1 - b0, cap_b, qc, code, b0, body_leaves[b], depth);
+        if (cut) {
+            body_cuts[b] = std::move(body_leaves[b]);
+            body_leaves[b].assign(1, b1);
+        }
     });
+    for (const auto &v : body_cuts) P.cut_end.insert(P.cut_end.end(), v.begin(), v.end());
     for (const auto &v : body_leaves) leaf_end.insert(leaf_end.end(), v.begin(), v.end());
     P.old2new.resize(n);
     for (int64_t i = 0; i < n; i++) P.old2new[P.new2old[i]] = (int32_t)i;
@@ -851,6 +864,105 @@ std::string build_plan(const PlanInput &in, Plan &P) {
         P = Plan();
         return std::string("planning failed: ") + e.what();
     }
+}
+
+namespace {
+
+struct CutScratch {
+    PermuteScratch permute;
+    std::vector<int32_t> id;  // a number per entry of the whole tile
+    std::vector<int64_t> ip, isp;
+};
+
+// Piece [lo, hi) of tile t, with the slab order of order_tile.
+CutTile cut_tile(const Plan &P, int64_t t, int64_t lo, int64_t hi, int slot_bytes, CutScratch &S) {
+    CutTile C;
+    C.lo = lo;
+    C.hi = hi;
+    C.body = P.body_of_tile[t];
+    const int64_t m0 = P.tile_mass_off[t], e0 = P.tile_ent_off[t], nm = hi - lo;
+    const uint32_t a = (uint32_t)(lo - m0), b = (uint32_t)(hi - m0);
+    std::vector<int32_t> &id = S.id;
+    auto code_at = [&](int64_t m, int64_t j) {
+        const int64_t l = m - m0;
+        return P.inc[ell_index(P.warp_inc_off[P.tile_warp_off[t] + l / 32], (uint32_t)(l % 32), (uint32_t)j)];
+    };
+    // the entries its masses have, in the order of their springs
+    id.assign((size_t)(P.tile_ent_off[t + 1] - e0), -1);
+    S.ip.assign(1, 0);
+    S.isp.clear();
+    for (int64_t m = lo; m < hi; m++) {
+        for (int64_t j = 0; j < P.deg[m]; j++) {
+            const int64_t e = code_at(m, j) & 0x7fffu;
+            id[(size_t)e] = 0;
+            S.isp.push_back(e0 + e);
+        }
+        S.ip.push_back((int64_t)S.isp.size());
+    }
+    std::vector<int64_t> part[2];  // actuated, others
+    for (size_t e = 0; e < id.size(); e++) {
+        if (id[e] < 0) continue;
+        part[(int64_t)e < P.tile_nact[t] ? 0 : 1].push_back(e0 + (int64_t)e);
+        const uint32_t w = P.ent_ends[e0 + e];
+        for (const uint32_t s : {w & 0xfffu, (w >> 12) & 0xfffu})
+            if (s < a || s >= b) C.halo.push_back((int32_t)(m0 + s));
+    }
+    for (auto &v : part)
+        std::sort(v.begin(), v.end(), [&](int64_t x, int64_t y) { return P.ent_spring[x] < P.ent_spring[y]; });
+    std::sort(C.halo.begin(), C.halo.end());
+    C.halo.erase(std::unique(C.halo.begin(), C.halo.end()), C.halo.end());
+    C.nh = (int32_t)C.halo.size();
+    C.nact = (int32_t)part[0].size();
+    auto slot = [&](uint32_t s) -> uint32_t {
+        if (s >= a && s < b) return s - a;
+        return (uint32_t)(nm + (std::lower_bound(C.halo.begin(), C.halo.begin() + C.nh, (int32_t)(m0 + s)) - C.halo.begin()));
+    };
+    bank_order_slab(part[0], part[1], slot_bytes, [&](int64_t e) { return slot(P.ent_ends[e] & 0xfffu); },
+                    [&](int64_t e) { return slot((P.ent_ends[e] >> 12) & 0xfffu); });
+    gather_permute(part[0], part[1], 0, nm, S.ip, S.isp, 255, S.permute);
+    for (const auto &v : part)
+        for (const int64_t e : v) {
+            id[(size_t)(e - e0)] = (int32_t)C.entry.size();
+            C.entry.push_back((int32_t)e);
+            const uint32_t w = P.ent_ends[e];
+            C.ends.push_back(pack_ends(slot(w & 0xfffu), slot((w >> 12) & 0xfffu), w >> 24));
+        }
+    while (C.halo.size() % 4) C.halo.push_back(C.halo.back());
+    for (int64_t w0 = lo; w0 < hi; w0 += 32) {
+        const int64_t w1 = std::min(w0 + 32, hi);
+        int64_t width = 0;
+        for (int64_t m = w0; m < w1; m++) width = std::max<int64_t>(width, P.deg[m]);
+        width = (width + 3) & ~int64_t(3);
+        const uint32_t off = (uint32_t)C.inc.size();
+        C.warp_inc.push_back(off);
+        C.inc.resize(C.inc.size() + (size_t)(width * 32), (uint16_t)C.entry.size());
+        for (int64_t m = w0; m < w1; m++)
+            for (int64_t j = 0; j < P.deg[m]; j++) {
+                const uint16_t c = code_at(m, j);
+                C.inc[ell_index(off, (uint32_t)(m - w0), (uint32_t)j)] = (uint16_t)(id[c & 0x7fffu] | (c & 0x8000u));
+            }
+    }
+    return C;
+}
+
+}  // namespace
+
+std::vector<CutTile> cut_tiles(const Plan &P, const std::vector<int64_t> &tiles, int slot_bytes) {
+    std::vector<std::array<int64_t, 3>> part;  // tile, lo, hi
+    for (const int64_t t : tiles) {
+        int64_t lo = P.tile_mass_off[t];
+        const int64_t hi = P.tile_mass_off[t + 1];
+        for (auto it = std::upper_bound(P.cut_end.begin(), P.cut_end.end(), lo); it != P.cut_end.end() && *it < hi; ++it) {
+            part.push_back({t, lo, *it});
+            lo = *it;
+        }
+        part.push_back({t, lo, hi});
+    }
+    std::vector<CutTile> out(part.size());
+    parallel_items<CutScratch>((int64_t)part.size(), 8, [&](CutScratch &S, int64_t q) {
+        out[q] = cut_tile(P, part[q][0], part[q][1], part[q][2], slot_bytes, S);
+    });
+    return out;
 }
 
 void build_resident(const PlanInput &in, const Plan &P, int max_masses, int bin_cap, ResPlan &R) {

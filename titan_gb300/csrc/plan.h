@@ -30,6 +30,7 @@ struct PlanInput {
     int tile_cap = 512;                  // masses per tile
     int tile_min = 32;                   // smallest tile_cap taken (smaller only by the engine's own choice)
     int whole_cap = 0;                   // bodies of at most this many masses stay one tile (0: tile_cap)
+    int cut_above = 0;                   // of those, the masses of bodies above this size keep the order of tiles of tile_cap (0: none)
     int slot_cap = 4095;                 // tile + halo slots per tile (12-bit)
     int entry_cap = 32767;               // slab entries per tile (15-bit)
     int heavy_threshold = 96;            // degree above this: warp-cooperative
@@ -73,6 +74,7 @@ struct Plan {
     std::vector<uint16_t> heavy_local;       // tile-local index of each heavy mass
     std::vector<uint32_t> heavy_inc_off;     // nheavy+1, into heavy_inc
     std::vector<uint16_t> heavy_inc;
+    std::vector<int64_t> cut_end;            // ends of the cuts of bodies kept whole (PlanInput::cut_above), ascending
     int64_t valid_springs = 0;
     int max_nm = 0, max_slots = 0, max_entries = 0, max_heavy = 0;
 };
@@ -80,6 +82,22 @@ struct Plan {
 // Returns "" on success, otherwise the reason (e.g. a mass whose degree does
 // not fit one tile's slab, or host memory exhausted); throws nothing.
 std::string build_plan(const PlanInput &in, Plan &out);
+
+// A piece of a tile without halo: masses [lo, hi) of it with the slab, halo
+// and incidence lists that a tile of its own would have.  halo: new mass indices, padded to a multiple of 4 as in
+// Plan; entry: the plan's entry behind each slab entry; warp_inc: block
+// offsets into inc.
+struct CutTile {
+    int64_t lo = 0, hi = 0;
+    int32_t body = 0, nh = 0, nact = 0;
+    std::vector<int32_t> halo, entry;
+    std::vector<uint32_t> ends, warp_inc;
+    std::vector<uint16_t> inc;
+};
+
+// The pieces, at P.cut_end, of the given tiles of P (no halo, no heavy
+// masses), in order; slot_bytes as in PlanInput.
+std::vector<CutTile> cut_tiles(const Plan &P, const std::vector<int64_t> &tiles, int slot_bytes);
 
 // Body-resident plan: bodies small enough for one CTA keep their state in
 // shared memory for a whole multi-step launch.  Whole bodies are packed into

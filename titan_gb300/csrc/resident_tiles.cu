@@ -195,6 +195,7 @@ __global__ void __launch_bounds__(512) k_tile_resident(StepArgs a, TileResArgs r
             T = T + prm->dt;
         }
 
+        if (r.time && t == 0 && threadIdx.x == 0) *r.time = T;
         const uint8_t *fin = (nsteps & 1) ? st1 : st0;
         for (int i = threadIdx.x; i < nm; i += blockDim.x) {
 #pragma unroll

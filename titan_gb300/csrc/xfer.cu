@@ -160,6 +160,27 @@ __global__ void __launch_bounds__(256) k_entries(EntryArgs a) {
     }
 }
 
+// One thread per repeated entry: its source's record and actuation record, the
+// entry word's type bits with the ends given.
+template <int PREC>
+__global__ void __launch_bounds__(256) k_repeat_entries(RepeatArgs a) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= a.count) return;
+    constexpr int kVec = PREC == P_FP64 ? 2 : 1;
+    float4 *const rec = reinterpret_cast<float4 *>(a.rec), *const act = reinterpret_cast<float4 *>(a.act);
+    const int64_t from = (int64_t)a.src[e] * kVec, to = (a.first + e) * kVec;
+#pragma unroll
+    for (int v = 0; v < kVec; v++) {
+        float4 r = rec[from + v];
+        // the entry word: FP64 the low half of the last double, FP32 the first float
+        float &w = PREC == P_FP64 ? r.z : r.x;
+        if (v == kVec - 1)
+            w = __uint_as_float((__float_as_uint(w) & 0xff000000u) | (a.ends[e] & 0x00ffffffu));
+        rec[to + v] = r;
+        act[to + v] = act[from + v];
+    }
+}
+
 // ------------------------------------------------------ diagnostics -------
 // Pass 1: each of kDiagBlocks blocks sums a fixed grid-stride share in FP64
 // and reduces it with a fixed tree; pass 2 reduces the partials the same way.
@@ -305,6 +326,17 @@ cudaError_t launch_entries(int precision, const EntryArgs &a, cudaStream_t s) {
         case P_FP64: k_entries<P_FP64><<<blocks, 256, 0, s>>>(a); break;
         case P_FP32: k_entries<P_FP32><<<blocks, 256, 0, s>>>(a); break;
         default: k_entries<P_FP32C><<<blocks, 256, 0, s>>>(a); break;
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_repeat_entries(int precision, const RepeatArgs &a, cudaStream_t s) {
+    if (a.count <= 0) return cudaSuccess;
+    const unsigned blocks = (unsigned)((a.count + 255) / 256);
+    switch (precision) {
+        case P_FP64: k_repeat_entries<P_FP64><<<blocks, 256, 0, s>>>(a); break;
+        case P_FP32: k_repeat_entries<P_FP32><<<blocks, 256, 0, s>>>(a); break;
+        default: k_repeat_entries<P_FP32C><<<blocks, 256, 0, s>>>(a); break;
     }
     return cudaGetLastError();
 }
