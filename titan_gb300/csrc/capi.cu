@@ -307,7 +307,8 @@ bool host_pinned(const void *p) {
 // here: 15 MB of velocities into a new array took 1.39 ms with pieces of 8 MB).
 void par_memcpy(void *dst, const void *src, size_t bytes) {
     constexpr size_t kPiece = 2u << 20;
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+    // (asked once: the answer takes 6 us)
+    static const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     const size_t nt = std::min<size_t>(std::min<size_t>(8, hw), (bytes + kPiece - 1) / kPiece);
     if (nt <= 1) {
         std::memcpy(dst, src, bytes);
@@ -959,43 +960,67 @@ std::string plan_scene(titan_gb300_sim *s, int tile_masses, tg::PlanInput &in) {
     return why;
 }
 
-// The device's copy of spring parameter q brought up to date with host.
-int upload_spring_array(titan_gb300_sim *s, int q, const std::vector<double> &host) {
-    cudaError_t e = cudaSuccess;
-    if (!s->d_sp[q] && !(s->d_sp[q] = (double *)s->mem.get(std::max<size_t>(1, host.size()) * 8, e)))
-        return s->cuda_fail(e, "alloc spring parameters");
-    if (!s->sp_current[q] && !host.empty())
-        CK(cudaMemcpyAsync(s->d_sp[q], host.data(), host.size() * 8, cudaMemcpyHostToDevice, s->stream),
-           "upload spring parameters");
-    s->sp_current[q] = true;
+// Device arrays for the spring parameters of mask (a bit per SP_*), in one
+// allocation (an allocation each took 10 us of a first update).
+bool alloc_spring_arrays(titan_gb300_sim *s, unsigned mask, cudaError_t &e) {
+    const size_t each = (std::max<size_t>(1, (size_t)s->ns) + 31) / 32 * 32;
+    int missing = 0;
+    for (int q = 0; q < titan_gb300_sim::SP_COUNT; q++) missing += (mask >> q & 1) && !s->d_sp[q];
+    if (!missing) return true;
+    double *p = (double *)s->mem.get(missing * each * 8, e);
+    if (!p) return false;
+    for (int q = 0; q < titan_gb300_sim::SP_COUNT; q++)
+        if ((mask >> q & 1) && !s->d_sp[q]) {
+            s->d_sp[q] = p;
+            p += each;
+        }
+    return true;
+}
+
+// The device's copies of the parameters of mask brought up to date with the
+// host arrays.
+int upload_spring_arrays(titan_gb300_sim *s, unsigned mask) {
+    const std::vector<double> *host[] = {&s->k, &s->rest, &s->damping, &s->omega, &s->amp, &s->phase};
+    for (int q = 0; q < titan_gb300_sim::SP_COUNT; q++) {
+        if (!(mask >> q & 1)) continue;
+        if (!s->sp_current[q] && !host[q]->empty())
+            CK(cudaMemcpyAsync(s->d_sp[q], host[q]->data(), host[q]->size() * 8, cudaMemcpyHostToDevice, s->stream),
+               "upload spring parameters");
+        s->sp_current[q] = true;
+    }
     return TITAN_GB300_OK;
 }
 
-// The slab's records rewritten on the device for the parameters given (a bit
-// per SP_*), every spring's.  The host loop that builds all records and the
-// two copies it needs took 1.5 ms for the 137,000 springs of a 23^3 design.
-int refresh_entries(titan_gb300_sim *s, unsigned given) {
+// The slab's records rewritten on the device for the parameters given,
+// every spring's (the host loop took 1.5 ms for the 137,000 springs of a 23^3
+// design).  done: false where there is no memory for it.
+int refresh_entries(titan_gb300_sim *s, unsigned given, bool &done) {
     const tg::Plan &P = s->plan;
     cudaError_t e = cudaSuccess;
-    if (!s->d_espring) {
+    done = false;
+    bool room = alloc_spring_arrays(s, given, e);
+    if (room && !s->d_espring) {
         std::vector<int32_t> es(P.ent_spring.begin(), P.ent_spring.end());
-        if (!(s->d_espring = dev_copy(s, es, e))) return s->cuda_fail(e, "upload entry springs");
+        room = (s->d_espring = dev_copy(s, es, e)) != nullptr;
     }
-    const std::vector<double> *host[] = {&s->k, &s->rest, &s->damping, &s->omega, &s->amp, &s->phase};
+    if (!room) {
+        if (e != cudaErrorMemoryAllocation) return s->cuda_fail(e, "spring parameters");
+        cudaGetLastError();
+        return TITAN_GB300_OK;
+    }
+    if (int rc = upload_spring_arrays(s, given)) return rc;
     tg::EntryArgs x{};
     x.spring = s->d_espring;
     x.rec = const_cast<void *>(s->args.ent);
     x.act = const_cast<void *>(s->args.act);
     x.count = (int64_t)P.ent_spring.size();
-    for (int q = 0; q < titan_gb300_sim::SP_COUNT; q++) {
-        if (!(given >> q & 1)) continue;
-        if (int rc = upload_spring_array(s, q, *host[q])) return rc;
-        x.par[q] = s->d_sp[q];
-    }
+    for (int q = 0; q < titan_gb300_sim::SP_COUNT; q++)
+        if (given >> q & 1) x.par[q] = s->d_sp[q];
     CK(tg::launch_entries(s->prec, x, s->stream), "refresh entries");
     if (s->short_form.ready)
         if (int rc = refresh_short(s)) return rc;
     s->tables_written = true;
+    done = true;
     return TITAN_GB300_OK;
 }
 
@@ -2628,8 +2653,13 @@ int titan_gb300_set_spring_params(titan_gb300_sim *s, int64_t count, const int64
         s->drop_graphs();
         return build_device(s);
     }
-    // whole arrays and no new types: the device rewrites the slab records
-    if (!idx && !retyped && !s->use_res && !s->use_pull) return given ? refresh_entries(s, given) : TITAN_GB300_OK;
+    if (!given && !retyped) return TITAN_GB300_OK;
+    // no new types: the device rewrites the slab records
+    if (!retyped && !s->use_res && !s->use_pull) {
+        bool done = false;
+        const int rc = refresh_entries(s, given, done);
+        if (rc || done) return rc;
+    }
     // type changes within passive or within active keep the slab order, but
     // the type bits live in the entry words
     if (type) {
@@ -2669,8 +2699,9 @@ int titan_gb300_diagnostics(titan_gb300_sim *s, double g_mag, double energy[4], 
         if (!(s->d_dout = (double *)s->mem.get(tg::kDiagQ * 8, e))) return s->cuda_fail(e, "diag alloc");
     }
     // (the host arrays change only after a wait for this stream)
-    if (int rc = upload_spring_array(s, titan_gb300_sim::SP_K, s->k)) return rc;
-    if (int rc = upload_spring_array(s, titan_gb300_sim::SP_REST, s->rest)) return rc;
+    constexpr unsigned kLengths = 1u << titan_gb300_sim::SP_K | 1u << titan_gb300_sim::SP_REST;
+    if (!alloc_spring_arrays(s, kLengths, e)) return s->cuda_fail(e, "diag alloc");
+    if (int rc = upload_spring_arrays(s, kLengths)) return rc;
     tg::DiagArgs d{};
     d.state = s->parity ? s->args.state1 : s->args.state0;
     d.mass = s->args.mass;
