@@ -251,13 +251,18 @@ int titan_gb300_resident_info(const titan_gb300_sim *sim, int64_t out[8]);
 
 /* One iteration of the reference's execute() loop body (src/sim.cu:1569-1590)
  * nsteps times: spring forces + mass update fused into one kernel per step,
- * replayed from cached CUDA graphs.  Asynchronous. */
+ * replayed from cached CUDA graphs, or (set_kernel 0) one launch of all tiles
+ * for up to 512 steps.  Asynchronous.  While the caller captures the handle's
+ * stream, single steps can be captured; a call of several steps on a scene
+ * with per-step tiles cannot, because it replays graphs. */
 int titan_gb300_step(titan_gb300_sim *sim, int64_t nsteps);
 
 /* Extension (no counterpart in the reference, whose execute() loop launches
  * kernels directly): builds and caches the CUDA graphs that step(nsteps)
  * would replay from the current step parity, without launching anything, so
- * that a later step(nsteps) spends no host time on graph capture.  Graphs
+ * that a later step(nsteps) spends no host time on graph capture; where one
+ * launch takes all tiles there is nothing to build (start and set_integrator
+ * have its kernel ready).  Graphs
  * are dropped when the scene is rebuilt (integrator switch, topology change).
  * On scenes of many bodies that longer calls keep resident it makes the tables
  * for calls of nsteps, if these are few, which step() makes at the 65th such

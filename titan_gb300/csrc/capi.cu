@@ -991,6 +991,21 @@ int upload_spring_arrays(titan_gb300_sim *s, unsigned mask) {
     return TITAN_GB300_OK;
 }
 
+// The resident grid's kernels for the current integrator made ready, so that
+// step() only launches; not used where the device cannot take all its CTAs at
+// once (the per-step kernels serve then, with the same tiles).
+int prepare_grid(titan_gb300_sim *s) {
+    if (!s->use_grid) return TITAN_GB300_OK;
+    int per_sm = 0;
+    CK(tg::grid_resident_prepare(s->prec, s->integrator, s->gargs, s->grid_shape, s->grid_smem, &per_sm),
+       "prepare resident grid");
+    if ((int64_t)s->gargs.ntiles > (int64_t)per_sm * sm_count(s)) s->use_grid = false;
+    if (s->single_shape >= 0)
+        CK(tg::grid_resident_prepare(s->prec, s->integrator, s->gargs, s->single_shape, s->grid_smem, &per_sm),
+           "prepare resident grid");
+    return TITAN_GB300_OK;
+}
+
 // The slab's records rewritten on the device for the parameters given,
 // every spring's (the host loop took 1.5 ms for the 137,000 springs of a 23^3
 // design).  done: false where there is no memory for it.
@@ -1393,6 +1408,7 @@ int build_device(titan_gb300_sim *s) {
         s->gargs.xbytes = np * tg::grid_resident_exchange_bytes(s->prec);
         if (!(s->gargs.xbuf = (uint8_t *)s->mem.get(2 * s->gargs.xbytes, e))) return s->cuda_fail(e, "alloc exchange");
         CK(cudaMemset(s->gargs.xbuf, 0, 2 * s->gargs.xbytes), "clear exchange");
+        if (int rc = prepare_grid(s)) return rc;
     }
     DEVCOPY(a.warp_inc_off, P.warp_inc_off, "upload warp offsets");
     std::vector<uint8_t> deg(np, 0);
@@ -2085,6 +2101,7 @@ int titan_gb300_set_integrator(titan_gb300_sim *s, int kind) try {
         CK(tg::step_ws_prepare(s->prec, kind, (size_t)s->args.ws.total), "set shared memory");
     else if (!s->use_async)
         CK(tg::step_prepare(s->prec, s->step_variant, kind, s->smem), "set shared memory");
+    if (int rc = prepare_grid(s)) return rc;
     return upload_params(s);
 } catch (...) {
     return host_exception(s);

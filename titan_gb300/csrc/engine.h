@@ -295,6 +295,9 @@ int grid_resident_threads(int shape);
 int grid_resident_ctas(int shape);
 int grid_resident_exchange_bytes(int precision);
 bool grid_resident_lanes(int precision, int shape, int max_nm);  // a lane per component (epilogue_lanes.cuh)
+// Raises the kernel's shared-memory limit, loads its code, and says how many of
+// its CTAs an SM takes.
+cudaError_t grid_resident_prepare(int precision, int integ, const GridResArgs &r, int shape, size_t smem, int *ctas_per_sm);
 cudaError_t launch_grid_resident(int precision, int integ, const StepArgs &a, const GridResArgs &r, int shape,
                                  size_t smem, int parity, int64_t nsteps, int write_acc, cudaStream_t s);
 // One pass (RK2: half `half` of a step) as an ordinary launch, FP32 forms;
