@@ -204,6 +204,11 @@ int titan_gb300_set_kernel(titan_gb300_sim *sim, int variant);
  * memory per CTA (bytes) -- of the resident-tile launch for form 5. */
 int titan_gb300_kernel_info(const titan_gb300_sim *sim, int64_t out[4]);
 
+/* How often a wait for another tile's masses is polled, where one launch
+ * takes all tiles, before the kernel gives up (TITAN_GB300_ETIMEOUT; see
+ * synchronize).  0: the default, 2^23, seconds.  At any time. */
+int titan_gb300_set_wait_limit(titan_gb300_sim *sim, int64_t polls);
+
 /* After start(): how calls of step() run that all tiles take at once
  * (set_kernel 0).  out[0] 1 when the scene has that form, else out[0..6] are 0;
  * out[1] tiles, a CTA each; out[2] threads per CTA; out[3] dynamic shared
@@ -271,9 +276,12 @@ int titan_gb300_prepare_steps(titan_gb300_sim *sim, int64_t nsteps);
 
 /* Wait for queued work; replaces the cudaDeviceSynchronize at src/sim.cu:1570.
  * TITAN_GB300_ETIMEOUT from here, poll or wait (not wait's own time limit)
- * means a step kernel's bounded wait for its shared-memory copies gave up:
- * the kernel stopped early, so the scene's state is undefined and the
- * handle must be destroyed. */
+ * means a step kernel's bounded wait (for its shared-memory copies, or for the
+ * masses of other tiles where one launch takes all of them) gave up: the
+ * kernel stopped early, so the scene's state is undefined.  step() then
+ * returns TITAN_GB300_ETIMEOUT until set_mass_state has uploaded all masses'
+ * positions and velocities (the time and the step count are those of the
+ * calls made; set_time), or the handle is destroyed. */
 int titan_gb300_synchronize(titan_gb300_sim *sim);
 
 /* step() is the asynchronous rollout launch.  poll(): TITAN_GB300_OK when

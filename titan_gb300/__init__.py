@@ -68,6 +68,7 @@ _SIGS = {
     "titan_gb300_set_kernel": (ctypes.c_int, [_P, ctypes.c_int]),
     "titan_gb300_set_occupancy": (ctypes.c_int, [_P, ctypes.c_int]),
     "titan_gb300_kernel_info": (ctypes.c_int, [_P, _I64]),
+    "titan_gb300_set_wait_limit": (ctypes.c_int, [_P, ctypes.c_int64]),
     "titan_gb300_grid_info": (ctypes.c_int, [_P, _I64]),
     "titan_gb300_set_resident": (ctypes.c_int, [_P, ctypes.c_int, ctypes.c_int, ctypes.c_int]),
     "titan_gb300_resident_info": (ctypes.c_int, [_P, _I64]),
@@ -332,6 +333,11 @@ class Sim:
         names = {1: "per-tile", 3: "per-tile-async", 4: "warp-specialised", 5: "resident-tiles", 6: "pull"}
         return {"kernel": names.get(int(out[0]), "per-tile"), "ctas": int(out[1]), "threads": int(out[2]),
                 "smem_bytes": int(out[3])}
+
+    def set_wait_limit(self, polls: int = 0):
+        """Polls of one wait for another tile's masses before a step kernel
+        gives up (error 6 from synchronize); 0: the default, seconds."""
+        self._check(self._L.titan_gb300_set_wait_limit(self._h, int(polls)), "set_wait_limit")
 
     def grid_info(self) -> dict:
         """How calls of step() run that all tiles take at once; last: the

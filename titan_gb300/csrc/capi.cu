@@ -132,6 +132,10 @@ struct titan_gb300_sim {
     double *d_sp[SP_COUNT] = {};
     bool sp_current[SP_COUNT] = {};
     int32_t *d_espring = nullptr;
+    int64_t wait_polls = 0;  // of one halo wait in the resident grid (0: the default)
+    // a step kernel gave up a wait: steps are refused until all positions and
+    // velocities are uploaded again
+    bool torn = false;
     // a kernel that writes the slab records may still run: the next step
     // kernel, which reads them before its grid_dep_wait(), must not start early
     bool tables_written = false;
@@ -1385,6 +1389,7 @@ int build_device(titan_gb300_sim *s) {
     }
     DEVCOPY(a.halo, P.halo, "upload halo");
     s->gargs = tg::GridResArgs{};
+    s->gargs.last_poll = (s->wait_polls > 0 ? (uint32_t)s->wait_polls : tg::kGridPolls) - 1;
     s->single_shape = -1;
     s->grid_last = 0;
     s->use_grid = !tiles_run.empty() && grid_wanted(s) && !s->use_pull &&
@@ -1619,7 +1624,9 @@ int check_kernel_error(titan_gb300_sim *s) {
     CK(cudaMemcpy(&flag, s->d_err, sizeof(int), cudaMemcpyDeviceToHost), "read error flag");
     if (flag) {
         cudaMemset(s->d_err, 0, sizeof(int));
-        return s->fail(TITAN_GB300_ETIMEOUT, "a step kernel's bounded wait for its shared-memory copies timed out");
+        s->torn = true;
+        return s->fail(TITAN_GB300_ETIMEOUT,
+                       "a step kernel's bounded wait (for its shared-memory copies or for other tiles' masses) timed out");
     }
     return TITAN_GB300_OK;
 }
@@ -1634,6 +1641,7 @@ int serve_begin(titan_gb300_sim *s, int device, int precision, size_t tile_smem,
     if (s->device != device || s->prec != precision)
         return why = "the scene's device or precision differs from the server's", TITAN_GB300_EINVAL;
     if (s->integrator != INTEG_EULER) return why = "the server steps symplectic Euler only", TITAN_GB300_EINVAL;
+    if (s->torn) return why = "the scene's state is undefined since a step kernel's wait timed out", TITAN_GB300_ETIMEOUT;
     if (s->use_res || s->use_rtiles || s->args.ntiles <= 0)
         return why = "start the scene with resident tiles and bins off (set_resident 0)", TITAN_GB300_EINVAL;
     size_t need = 0;
@@ -1808,6 +1816,14 @@ int titan_gb300_resident_info(const titan_gb300_sim *s, int64_t out[8]) {
     out[5] = s->res_threads;
     out[6] = s->res_ctas;
     out[7] = (int64_t)tg::resident_smem_bytes(s->prec, s->rargs.cap);
+    return TITAN_GB300_OK;
+}
+
+int titan_gb300_set_wait_limit(titan_gb300_sim *s, int64_t polls) {
+    if (!s) return TITAN_GB300_EINVAL;
+    if (polls < 0 || polls > (int64_t)UINT32_MAX) return s->fail(TITAN_GB300_EINVAL, "polls must be in [0, 2^32)");
+    s->wait_polls = polls;
+    s->gargs.last_poll = (polls > 0 ? (uint32_t)polls : tg::kGridPolls) - 1;
     return TITAN_GB300_OK;
 }
 
@@ -2189,6 +2205,8 @@ int titan_gb300_step(titan_gb300_sim *s, int64_t nsteps) try {
     if (s->serving) return s->fail(TITAN_GB300_ESTATE, "the scene is being stepped by a request server");
     if (!s->started) return s->fail(TITAN_GB300_ESTATE, "The simulation has not started.");
     if (nsteps < 0) return s->fail(TITAN_GB300_EINVAL, "negative step count");
+    if (s->torn)
+        return s->fail(TITAN_GB300_ETIMEOUT, "a step kernel's wait timed out: upload all positions and velocities first");
     if (nsteps == 0) return TITAN_GB300_OK;
     if (!ensure_device(s)) return s->fail(TITAN_GB300_ECUDA, "cudaSetDevice failed");
     cudaError_t e = cudaSuccess;
@@ -2614,6 +2632,10 @@ int titan_gb300_set_mass_state(titan_gb300_sim *s, int64_t count, const int64_t 
         x.ivel = vel ? s->d_xfer + 3 * count : nullptr;
         CK(tg::launch_scatter(s->prec, x, s->stream), "scatter");
         CK(cudaStreamSynchronize(s->stream), "set");
+        if (s->torn && !idx && pos && vel) {  // a whole state again; the time record, too
+            if (int rc = upload_params(s)) return rc;
+            s->torn = false;
+        }
     }
     return TITAN_GB300_OK;
 } catch (...) {

@@ -176,6 +176,7 @@ struct GridResArgs {
     int32_t stage;              // 1: slab, actuation and incidence records in shared memory
     int32_t half;               // RK2: the half step that the launch's first pass is
     int32_t single;             // a launch of one pass, by launch_grid_single
+    uint32_t last_poll;         // of one wait, counted from 0, before the kernel gives up
 };
 
 // Per-mass gather / scatter between caller order and tiled order.
@@ -290,6 +291,7 @@ cudaError_t launch_tile_resident(int precision, const StepArgs &a, const TileRes
 // bytes of one mass in an exchange buffer; and the cooperative launch of
 // nsteps steps.
 constexpr int kGridShapes = 3;
+constexpr uint32_t kGridPolls = 1u << 23;  // seconds
 size_t grid_resident_smem_bytes(int precision, const TileInfo &ti, int stage);
 int grid_resident_threads(int shape);
 int grid_resident_ctas(int shape);

@@ -61,7 +61,6 @@ struct GridShape {
 };
 constexpr GridShape kShapes[kGridShapes] = {{512, 1}, {256, 2}, {128, 4}};
 constexpr int kLaneWarps = 8;  // warps a tile's masses may take with a lane per component
-constexpr uint32_t kGridSpins = 1u << 23;  // polls of one wait: seconds
 
 __host__ __device__ constexpr int64_t rg_align16(int64_t x) { return (x + 15) & ~int64_t(15); }
 constexpr int64_t kParamBytes = (int64_t)sizeof(DevParams);  // a multiple of 16
@@ -303,9 +302,9 @@ __global__ void __launch_bounds__(kShapes[SHAPE].threads, kShapes[SHAPE].ctas)
                             dst[2] = x[k].w[2];
                             todo &= ~(1u << k);
                         }
-                    if (it == kGridSpins ||
+                    if (it == r.last_poll ||
                         ((it & 1023u) == 1023u && *reinterpret_cast<const volatile int *>(a.err))) {
-                        gave_up = true;
+                        gave_up = todo != 0;
                         break;
                     }
                 }
