@@ -161,7 +161,9 @@ int titan_gb300_start(titan_gb300_sim *sim, int tile_masses);
  * the same precision, kernel form, masses, springs (ends), fixed masses,
  * actuated springs and bodies -- positions, parameters and constraints may
  * differ.  The plan is used when start()'s requested tile size equals the
- * one src was planned with (0 for both: the default).  Results
+ * one src was planned with (0 for both: the default, and then only where this
+ * handle's integrator, launch shape and resident mode give the same default
+ * sizes; else start() plans).  Results
  * do not depend on which plan a scene runs with. */
 int titan_gb300_adopt_plan(titan_gb300_sim *sim, const titan_gb300_sim *src);
 

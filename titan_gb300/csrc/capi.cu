@@ -197,6 +197,9 @@ struct titan_gb300_sim {
     bool plan_adopted = false;
     int plan_tile = 0;  // tile size the current plan was built with
     int plan_req = 0;   // tile size requested for it (0: the default)
+    // sizes that the handle's settings asked the planner for: tile, smallest
+    // tile, whole bodies, cut
+    std::array<int, 4> plan_ask{};
 
     cudaError_t launch(int parity, int write_acc, int stage = 0) {
         if (args.ntiles == 0) return cudaSuccess;
@@ -599,6 +602,8 @@ int sm_count(const titan_gb300_sim *s) {
     return sms;
 }
 
+std::array<int, 4> plan_sizes(const tg::PlanInput &in) { return {in.tile_cap, in.tile_min, in.whole_cap, in.cut_above}; }
+
 // Whether nothing chose another form than the resident grid for calls of
 // several steps.
 bool grid_wanted(const titan_gb300_sim *s) {
@@ -940,6 +945,7 @@ int setup_pull(titan_gb300_sim *s, std::vector<tg::TileInfo> &tiles_run) {
 std::string plan_scene(titan_gb300_sim *s, int tile_masses, tg::PlanInput &in) {
     s->plan_req = tile_masses;
     in = plan_input(s, tile_masses, true);
+    s->plan_ask = plan_sizes(in);
     std::string why;
     if (in.tile_min < 32) {  // tiles for the resident grid, if it takes them (heavy masses may split tiles)
         int shape, stage;
@@ -1153,7 +1159,10 @@ int build_device(titan_gb300_sim *s) {
     s->free_device();
     tg::PlanInput in;
     const size_t rs = s->rsize();
-    if (s->plan_adopted && !s->started && s->plan_req == s->tile_masses) {
+    // (a default plan depends on the integrator and on the form and resident
+    // modes chosen: only one that these settings would ask for is taken)
+    if (s->plan_adopted && !s->started && s->plan_req == s->tile_masses &&
+        s->plan_ask == plan_sizes(plan_input(s, s->tile_masses, true))) {
         s->plan_adopted = false;  // the adopted plan serves this first start
         in = plan_input(s, s->plan_tile);
     } else {
@@ -1860,6 +1869,7 @@ int titan_gb300_adopt_plan(titan_gb300_sim *s, const titan_gb300_sim *src) try {
     s->plan = src->plan;
     s->plan_tile = src->plan_tile;
     s->plan_req = src->plan_req;
+    s->plan_ask = src->plan_ask;
     s->plan_adopted = true;
     return TITAN_GB300_OK;
 } catch (...) {
