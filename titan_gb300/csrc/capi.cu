@@ -1356,7 +1356,12 @@ int build_device(titan_gb300_sim *s) {
                 return s->fail(TITAN_GB300_EINVAL, "3 or 4 CTAs per SM need at most 256 threads per CTA");
             s->step_variant = s->min_ctas_req == 3 ? 1 : 2;
         }
-        if (s->prec == P_FP64 && s->threads <= 256 && (int64_t)tiles_run.size() > 2 * sms_dev) s->step_variant = 3;
+        // capped registers, which spill, only where three CTAs' shared memory
+        // fits an SM: 60^3 with tiles of 128 masses 222 us with the cap and 215
+        // without, of 192 302 and 278
+        const bool three = 3 * (s->smem + 1024) <= 228 * 1024;
+        if (s->prec == P_FP64 && s->threads <= 256 && three && (int64_t)tiles_run.size() > 2 * sms_dev)
+            s->step_variant = 3;
         if (s->use_async)
             CK(tg::step_async_prepare(s->prec, s->smem), "set shared memory");
         else
