@@ -16,13 +16,16 @@ from pathlib import Path
 from . import FP64, Sim
 from . import workloads as wl
 
-# (kernel form, tile masses, threads per CTA); form 6 = pull (threads =
+# (kernel form, tile masses, threads per CTA); (0, 0, 0) = the engine's own
+# choice, which no other candidate repeats (any form or launch shape turns the
+# resident grid off); form 6 = pull (threads =
 # consumer threads: a team of one warp per 32 tile masses per tile in
 # flight; 0 = two teams), 4 = warp-specialised (threads = consumer
 # threads), 3 = per-tile with asynchronous staging, 1 = per-tile
-CANDIDATES_F32 = [(6, 256, 0), (6, 192, 0), (6, 128, 0), (6, 128, 384), (4, 208, 448), (4, 192, 448),
+DEFAULT = (0, 0, 0)
+CANDIDATES_F32 = [DEFAULT, (6, 256, 0), (6, 192, 0), (6, 128, 0), (6, 128, 384), (4, 208, 448), (4, 192, 448),
                   (4, 160, 448), (3, 256, 256), (1, 256, 256), (1, 128, 128)]
-CANDIDATES_F64 = [(1, 128, 128), (1, 64, 128), (3, 128, 128), (1, 128, 256)]
+CANDIDATES_F64 = [DEFAULT, (1, 128, 128), (1, 64, 128), (3, 128, 128), (1, 128, 256)]
 
 
 def _default_cache() -> Path:
@@ -70,7 +73,9 @@ def autotune(sc: dict, precision: int, steps: int = 60, candidates=None, cache_p
             table = json.loads(cache.read_text())
         except ValueError:
             table = {}
-    if key in table and not refresh:
+    # (an entry of a list without the engine's own choice is timed again)
+    tried = [tuple(r["candidate"]) for r in table[key].get("tried", [])] if key in table else []
+    if key in table and not refresh and (candidates or DEFAULT in tried):
         return table[key]
     cands = candidates or (CANDIDATES_F64 if precision == FP64 else CANDIDATES_F32)
     results = []
