@@ -308,7 +308,9 @@ int titan_gb300_export_indices(titan_gb300_sim *sim, uint32_t *out, int out_on_d
 /* Replaces time() (src/sim.cu:1082): host-accumulated T (T += dt per step). */
 double titan_gb300_time(const titan_gb300_sim *sim);
 
-/* Device memory held by the handle (bytes), for admission control. */
+/* Device memory of the handle (bytes), for admission control: what it holds
+ * and what the first updates of its spring parameters will add (up to 48 bytes
+ * a spring and 4 a slab entry). */
 int64_t titan_gb300_device_bytes(const titan_gb300_sim *sim);
 
 /* Page-locked host memory (cudaMallocHost) for state buffers: get_state,

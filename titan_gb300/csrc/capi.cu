@@ -970,10 +970,21 @@ std::string plan_scene(titan_gb300_sim *s, int tile_masses, tg::PlanInput &in) {
     return why;
 }
 
+// Doubles of one spring parameter's device array.
+size_t spring_array_size(const titan_gb300_sim *s) { return (std::max<size_t>(1, (size_t)s->ns) + 31) / 32 * 32; }
+
+// Device memory that updates of all spring parameters will still take.
+size_t spring_update_bytes(const titan_gb300_sim *s) {
+    if (!s->started || s->use_res || s->use_pull) return 0;
+    size_t bytes = s->d_espring ? 0 : std::max<size_t>(16, s->plan.ent_spring.size() * sizeof(int32_t));
+    for (int q = 0; q < titan_gb300_sim::SP_COUNT; q++) bytes += s->d_sp[q] ? 0 : spring_array_size(s) * 8;
+    return bytes;
+}
+
 // Device arrays for the spring parameters of mask (a bit per SP_*), in one
 // allocation (an allocation each took 10 us of a first update).
 bool alloc_spring_arrays(titan_gb300_sim *s, unsigned mask, cudaError_t &e) {
-    const size_t each = (std::max<size_t>(1, (size_t)s->ns) + 31) / 32 * 32;
+    const size_t each = spring_array_size(s);
     int missing = 0;
     for (int q = 0; q < titan_gb300_sim::SP_COUNT; q++) missing += (mask >> q & 1) && !s->d_sp[q];
     if (!missing) return true;
@@ -2462,7 +2473,9 @@ int titan_gb300_export_indices(titan_gb300_sim *s, uint32_t *out, int out_on_dev
 
 double titan_gb300_time(const titan_gb300_sim *s) { return s ? s->T : 0.0; }
 
-int64_t titan_gb300_device_bytes(const titan_gb300_sim *s) { return s ? (int64_t)s->mem.total : 0; }
+int64_t titan_gb300_device_bytes(const titan_gb300_sim *s) {
+    return s ? (int64_t)(s->mem.total + spring_update_bytes(s)) : 0;
+}
 
 void *titan_gb300_host_alloc(size_t bytes) {
     void *p = nullptr;
