@@ -32,8 +32,9 @@
 // tiny values); the caller then uses the FP64 instructions.  A zero carries
 // an exponent far below any other through products and quotients.
 //
-// The host compiles the same functions (with its own initial estimates), so
-// that they are also tested on the CPU.
+// The host compiles the same functions, with its own initial estimates, for
+// the test against IEEE results and the C library's sine
+// (tests/test_fp64_alu_cpu.py).
 #pragma once
 
 #include <cstdint>
@@ -106,25 +107,6 @@ TG_HD uint64_t alu_mullo64(uint64_t a, uint64_t b) {
     const uint64_t p = (uint64_t)alu_lo(a) * alu_lo(b);
     return alu_join(alu_hi(p) + alu_lo(a) * alu_hi(b) + alu_hi(a) * alu_lo(b), alu_lo(p));
 }
-// 1/sqrt(x), 1/x, good to 22 bits
-TG_HD float alu_rsqrt_estimate(float x) {
-#ifdef __CUDA_ARCH__
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-#else
-    return 1.0f / std::sqrt(x);
-#endif
-}
-TG_HD float alu_rcp_estimate(float x) {
-#ifdef __CUDA_ARCH__
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-#else
-    return 1.0f / x;
-#endif
-}
 TG_HD uint32_t alu_float_bits(float x) {
 #ifdef __CUDA_ARCH__
     return __float_as_uint(x);
@@ -141,6 +123,32 @@ TG_HD float alu_float(uint32_t b) {
     float x;
     std::memcpy(&x, &b, 4);
     return x;
+#endif
+}
+#ifndef __CUDA_ARCH__
+// the host's estimates, moved by a number of units that a test chooses
+#ifndef TG_ALU_HOST_SHIFT
+#define TG_ALU_HOST_SHIFT 0
+#endif
+inline float alu_host_estimate(float y) { return alu_float(alu_float_bits(y) + (uint32_t)(TG_ALU_HOST_SHIFT)); }
+#endif
+// 1/sqrt(x), 1/x, good to 22 bits
+TG_HD float alu_rsqrt_estimate(float x) {
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+#else
+    return alu_host_estimate(1.0f / std::sqrt(x));
+#endif
+}
+TG_HD float alu_rcp_estimate(float x) {
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+#else
+    return alu_host_estimate(1.0f / x);
 #endif
 }
 
@@ -317,7 +325,7 @@ TG_HD Alu alu_sin(double x) {
     r = alu_mad(mh, k2, (uint64_t)alu_hi(hi) + alu_hi(r));
     const uint32_t w3 = alu_lo(r), w4 = alu_hi(r);
     // the 64 bits below the binary point: bit 1107 - e - 32 (of w1's lowest
-    // upwards) in [22, 75]
+    // upwards) in [23, 76]
     const uint32_t at = 1075u - e;
     const uint32_t v0 = at >= 64 ? w3 : (at >= 32 ? w2 : w1), v1 = at >= 64 ? w4 : (at >= 32 ? w3 : w2),
                    v2 = at >= 64 ? 0u : (at >= 32 ? w4 : w3);
