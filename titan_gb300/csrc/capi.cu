@@ -622,8 +622,11 @@ bool grid_wanted(const titan_gb300_sim *s) {
 // steps, 6.2 against 3.0 ms, 24 of 27 to 3,000, 190 steps, 12.8 against 9.8.
 // 128 threads: 9^3 7.5 us against 6.2.  The FP32 forms 128 up to 400 entries,
 // else 256 (16^3: 2.85 us with 128, 3.1 with 256; 24 scenes of 27 to 60,000
-// masses in flight together, 200 steps: 8.2 against 10.5 ms).  Returns false
-// when the tiles do not all fit.
+// masses in flight together, 200 steps: 8.2 against 10.5 ms).  128 threads in
+// FP64 and 512 in the FP32 forms are taken where the others refuse, which
+// with the default sizes they do not: tiles asked for by start() of more than
+// 256 masses (FP32), or of more than 304 in number (FP64).  Returns false when
+// the tiles do not all fit.
 bool choose_grid(const titan_gb300_sim *s, const std::vector<tg::TileInfo> &tiles, int &shape, int &stage, size_t &bytes) {
     size_t smem[2] = {0, 0};
     int max_nm = 0, max_ne = 0;
@@ -708,9 +711,10 @@ tg::PlanInput plan_input(titan_gb300_sim *s, int tile_masses, bool grid = false)
     // smaller tiles so that their tiles cover the SMs: FP64 about 1.6 tiles
     // per SM (tiles of 32 to 96 masses), the warp-specialised form about
     // 4 (64 to 208).  In the FP32 forms a body that fits the large-scene
-    // tile stays whole (a halo-free tile runs resident: 2.0 us per step for
-    // the 5^3 lattice against 3.3 split in four); in FP64, bound by each
-    // SM's FP64 pipe, it is split like the rest (5^3: 8.6 us in four tiles).
+    // tile stays whole (a halo-free tile runs resident on one SM: 2.00 us per
+    // step for the 5^3 lattice; in the resident grid as eight tiles of 16
+    // masses 1.83, as four of 32 2.01); in FP64, bound by each SM's FP64 pipe,
+    // it is split like the rest (5^3: 4.6 us in 16 tiles).
     // Measured on GB300, 20^3 lattice, per-step kernels: FP64 16.1 us per
     // step with 32-mass tiles; FP32C 5.3 us with 64 against 6.5 with 208.
     const bool pull = pull_wanted(s);
@@ -1319,7 +1323,8 @@ int build_device(titan_gb300_sim *s) {
     // automatic choice: the warp-specialised form in FP32 and FP32C (measured
     // fastest on GB300, see the kernel-form sweep in profiles/) when two of
     // the scene's tiles fit one SM's shared memory, else the per-tile form;
-    // the per-tile form in FP64 (FP64-ALU bound, no gain from overlap)
+    // the per-tile form in FP64, whose CTAs overlap each other instead (three
+    // per SM: 80^3 449 us per step against 496 with one)
     // the pull form when requested (or automatic, kPullAuto), else the
     // warp-specialised one
     s->use_pull = false;
@@ -2526,8 +2531,8 @@ int titan_gb300_get_masses(titan_gb300_sim *s, int64_t count, const int64_t *idx
         x.idx = s->d_idx;
     }
     // only the requested arrays come back: the kernel writes them into a
-    // caller buffer that is page-locked as a whole, else into the handle's staging buffer, and
-    // the error flag beside that
+    // caller buffer that is page-locked as a whole, else into the handle's
+    // staging buffer, and the error flag beside that
     double *outs[3] = {pos, vel, acc}, *dst[3] = {nullptr, nullptr, nullptr};
     bool direct[3] = {false, false, false};
     const bool any = pos || vel || acc;
