@@ -87,3 +87,27 @@ def test_repeated_short_calls_get_their_tables():
             assert s.grid_info()["last"] == (3 if resident is None and q >= 64 else 0)
         got.append(s.get_state(acc=True, T=True))
     same(*got)
+
+
+def test_mass_attributes_set_after_the_tables():
+    """The tables made before hold no copy of what later calls replace: masses,
+    loads and the arrays of local constraints, which are uploaded with them."""
+    sc = wl.robot_batch(310, side_range=(6, 7), seed=3)
+    n = sc["pos"].shape[0]
+    rng = np.random.default_rng(8)
+    on = rng.random(n) < 0.1
+    sc["lc_ptr"] = np.concatenate([[0], np.cumsum(on)]).astype(np.int64)
+    sc["lc_type"] = np.zeros(int(on.sum()), np.int32)
+    sc["lc_vec"] = np.tile([0.0, 0.0, 1.0], (int(on.sum()), 1))
+    sc["lc_num"] = np.full(int(on.sum()), 0.1)
+    ext, m = rng.normal(size=(n, 3)), rng.uniform(0.05, 0.2, n)
+    got = []
+    for resident in (None, (0, 0, 0)):
+        s = wl.make_sim(sc, tg.FP32C, resident=resident)
+        s.prepare_steps(1)
+        for q in range(3):
+            s.set_mass_state(None, ext=ext * q, m=m * (1 + q))
+            for c in (1, 1, 9, 1):
+                s.step(c)
+        got.append(s.get_state(acc=True, T=True))
+    same(*got)

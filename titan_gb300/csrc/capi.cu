@@ -1154,6 +1154,22 @@ int build_short(titan_gb300_sim *s) {
     return refresh_short(s);
 }
 
+// The step arguments with those tables (the rest as it is now: new local
+// constraints, for instance, have new arrays).
+tg::StepArgs short_args(const titan_gb300_sim *s) {
+    tg::StepArgs a = s->args;
+    const tg::StepArgs &t = s->short_form.args;
+    a.tiles = t.tiles;
+    a.halo = t.halo;
+    a.ent = t.ent;
+    a.act = t.act;
+    a.warp_inc_off = t.warp_inc_off;
+    a.inc = t.inc;
+    a.ntiles = t.ntiles;
+    a.ws = t.ws;
+    return a;
+}
+
 // Whether a call of nsteps runs in those tiles; makes their tables when there
 // have been enough such calls, or at once (now).
 bool short_runs(titan_gb300_sim *s, int64_t nsteps, bool now, int &rc) {
@@ -2259,8 +2275,9 @@ int titan_gb300_step(titan_gb300_sim *s, int64_t nsteps) try {
     }
     int rc_short = TITAN_GB300_OK;
     if (short_runs(s, nsteps, false, rc_short)) {
+        const tg::StepArgs a = short_args(s);
         for (int64_t i = 0; i < nsteps; i++) {
-            CK(tg::launch_step_ws(s->prec, s->integrator, s->short_form.args, s->short_form.ctas,
+            CK(tg::launch_step_ws(s->prec, s->integrator, a, s->short_form.ctas,
                                   tg::kWsMaxConsumerWarps, s->parity, i == nsteps - 1, s->stream, !s->tables_written),
                "launch step");
             s->tables_written = false;
