@@ -199,8 +199,9 @@ int titan_gb300_set_occupancy(titan_gb300_sim *sim, int min_ctas_per_sm);
  * start(). */
 int titan_gb300_set_kernel(titan_gb300_sim *sim, int variant);
 
-/* After start(): out[0] kernel form of the per-step launches (single steps
- * and what the one-launch form of set_kernel 0 does not hold) (1 to 4; 5
+/* After start(): out[0] kernel form of the per-step launches (what the
+ * one-launch form of set_kernel 0 and its single pass, grid_info, do not take)
+ * (1 to 4; 5
  * when resident tiles carry the whole scene and no per-step kernel runs),
  * out[1] CTAs per launch, out[2] threads per CTA, out[3] dynamic shared
  * memory per CTA (bytes) -- of the resident-tile launch for form 5. */
